@@ -132,6 +132,23 @@ def test_merge_attn_out_reference_accumulators(lse_dtype, new_dtype):
     assert lsed.dtype == lse_dtype
 
 
+@pytest.mark.parametrize("S,Dm", [(1, 128), (31, 64), (32, 128), (33, 100), (70, 4), (65, 68), (40, 160)])
+def test_merge_attn_out_row_remainders(S, Dm):
+    """The accumulator merge takes 32 tokens of a head per warp and 16 or 32 lanes per row: token counts and
+    head dimensions around those edges, with a result beyond the tokens that must stay as it is."""
+    from ring_swa.ops import merge_attn_out
+    g = torch.Generator().manual_seed(S + Dm)
+    acc, new = torch.randn(1, S + 3, 2, Dm, generator=g), torch.randn(1, S, 2, Dm, generator=g).bfloat16()
+    lse, new_lse = torch.randn(1, 2, S + 3, generator=g) * 3, torch.randn(1, 2, S, generator=g) * 3
+    ro, rl = _torch_merge(acc[:, :S], lse[:, :, :S], new.float(), new_lse)
+    accd, lsed = acc.to(_dev()), lse.to(_dev())
+    merge_attn_out(accd[:, :S], lsed[:, :, :S], new.to(_dev()), new_lse.to(_dev()))
+    assert torch.equal(accd[:, S:].cpu(), acc[:, S:]) and torch.equal(lsed[:, :, S:].cpu(), lse[:, :, S:])
+    # float32 arithmetic of three operations around two exponentials: a few 2^-22
+    assert_close("merged out", accd[:, :S], ro.float(), atol=1e-5, rtol=1e-5, rel_l2=1e-5)
+    assert_lse_close(lsed[:, :, :S], rl.float(), tol=1e-5)
+
+
 def test_flash_attn_funcs_accumulate_like_the_reference_loop():
     """Two partial results over disjoint key blocks merged through flash_attn_fwd_func equal attention
     over all keys; flash_attn_bwd_func with the final out / lse gives each block's gradients."""
