@@ -144,6 +144,12 @@ typedef struct rswa_bwd_params {
 } rswa_bwd_params_t;
 
 int64_t rswa_bwd_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_q_heads, int32_t head_dim);
+/* Further bytes of workspace, behind the ones above, with which a call with sink tokens runs faster: the
+ * queries beyond the window of a sink token are then worked on in parallel, and partial sums of the
+ * sink rows' gradients are kept there.  0 where they would not be used; without them the call is
+ * correct all the same.  n_seqs: 0 without cu_seqlens. */
+int64_t rswa_bwd_sink_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_kv_heads, int32_t window,
+                                      int32_t n_sink, int32_t n_seqs);
 int rswa_bwd(const rswa_bwd_params_t* p, void* stream);
 
 /* The whole backward for callers that cannot allocate device memory: same inputs, outputs and

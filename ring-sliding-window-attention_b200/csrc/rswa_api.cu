@@ -202,6 +202,30 @@ int sm_count() {
   return cached[dev];
 }
 
+// How the dK/dV kernel treats sink tokens (see BwdKernelParams).  A key tile that holds one is seen by all later
+// query tiles of its sequence, one after the other in one CTA: on 16000 tokens of 32/4 heads with a window of
+// 1000 that chain of 1000 tile products was 1.7 of the kernel's 1.75 ms.  The queries beyond the window are cut
+// into segments instead, each about as long as an ordinary key tile's item (`per_key` query tiles), so that no
+// item is longer than the others.  Left alone: calls short enough for the chain to be at most twice an
+// ordinary item (the partial sums cost another launch), very many sink tokens (the partial sums are kept per
+// sink token) and packs of sequences shorter than a tile on average (their segments would be mostly empty).
+struct FarPlan {
+  int segs, chunk, slots;
+  int64_t bytes;
+};
+static FarPlan far_plan(int batch, int q_len, int hkv, int window, int n_sink, int n_seqs) {
+  FarPlan f = {0, 0, 0, 0};
+  const int n_tiles = (q_len + kTile - 1) / kTile;
+  const int per_key = window / kTile + 2;
+  if (n_sink <= 0 || n_sink > 16 || n_tiles / 2 < per_key || n_seqs > n_tiles) return f;
+  const int chunk_tiles = per_key > 4 ? per_key : 4;
+  f.chunk = chunk_tiles * kTile;
+  f.segs = (n_tiles + chunk_tiles - 1) / chunk_tiles + n_seqs;
+  f.slots = f.segs + (n_seqs > 0 ? n_seqs + 1 : 1);
+  f.bytes = static_cast<int64_t>(batch) * hkv * f.slots * n_sink * 2 * kHeadDim * sizeof(float);
+  return f;
+}
+
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace rswa
@@ -271,6 +295,12 @@ extern "C" int64_t rswa_bwd_workspace_bytes(int32_t batch, int32_t q_len, int32_
   // two fp32 rows per (batch, head): delta = rowsum(dO * O) and lse * log2(e), padded to whole tiles;
   // then 256 bytes that hold the work counters of the dQ and dK/dV kernels
   return 2 * static_cast<int64_t>(batch) * n_q_heads * q_len_pad * 4 + 256;
+}
+
+extern "C" int64_t rswa_bwd_sink_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_kv_heads, int32_t window,
+                                                 int32_t n_sink, int32_t n_seqs) {
+  if (batch <= 0 || q_len <= 0 || n_kv_heads <= 0 || window < 0 || n_sink < 0 || n_seqs < 0) return -1;
+  return far_plan(batch, q_len, n_kv_heads, window, n_sink, n_seqs).bytes;
 }
 
 extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
@@ -378,6 +408,13 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   }
   kk.span_tile0[n_k] = total_tiles;
   kk.n_spans = n_k;
+  const FarPlan far = far_plan(g.batch, g.q_len, g.n_kv_heads, g.window, g.n_sink, g.cu_seqlens ? g.n_seqs : 0);
+  if (far.bytes > 0 && n_k > 0 && p->workspace_bytes >= need + far.bytes) {
+    kk.far_segs = far.segs;
+    kk.far_chunk = far.chunk;
+    kk.far_slots = far.slots;
+    kk.far_ws = reinterpret_cast<float*>(static_cast<uint8_t*>(p->workspace) + need);
+  }
 
   if (p->flags & RSWA_BWD_INIT) {
     rc = launch_delta(*p, delta, lse2, q_len_pad, stream);

@@ -60,6 +60,8 @@ constexpr bool kBwdPoly = RSWA_BWD_POLY != 0;  // a quarter of the exponentials 
 struct BwdItemGeom {
   int valid;  // 0: no more work
   int b, hk, sp, key0, n_valid_k, t0, qt_first, n_qt;
+  int far;    // segment of a far item + 1; 0: an ordinary key tile
+  int far_hi; // last query position of a far item
 };
 
 struct BwdCtl {
@@ -153,6 +155,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
       int nk = 0;  // items with work so far
       for (int n = 0;; ++n) {
         const int slot = n & 1;
+        // (waiting for the same phase again, after an item that turned out to be empty, returns at once)
         if (n >= 2 && !mbar_wait<200>(&ctl->geom_free[slot], ((n >> 1) - 1) & 1, err, kErrWaitProducer)) break;
         BwdItemGeom* g = &ctl->geom[slot];
         // work item: batch row fastest, then KV head, then key tile (tiles of the first span first)
@@ -168,24 +171,44 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         const int b = idx % p.batch;
         idx /= p.batch;
         const int hk = idx % p.hkv;
-        const int kt_g = idx / p.hkv;
-        int sp = 0;
-        while (sp + 1 < n_spans && kt_g >= p.span_tile0[sp + 1]) ++sp;
-        const int key0 = (kt_g - p.span_tile0[sp]) * kTile;  // token offset inside the span
-        const int n_valid_k = min(kTile, p.span_len[sp] - key0);
-        const int t0 = p.span_pos[sp] + key0;
-        // query tiles that can see at least one key of this tile
-        const int t_last = t0 + n_valid_k - 1;
-        int s_last, e_last;
-        seq_of(cu_seq, n_seqs, t_last, s_last, e_last);
-        int pmax;
-        if (n_sink > 0 && s_last + n_sink > t0) {
-          pmax = e_last - 1;  // the tile holds a sink token: every later query of that sequence
+        idx /= p.hkv;
+        int sp = 0, key0, n_valid_k, t0, q_lo, q_hi, far = 0;
+        if (!kPlain && idx < p.far_segs * n_spans) {
+          // The queries of one segment beyond the window of the sink tokens of their sequence: a tile that
+          // starts at the first of those this span holds (a TMA load may start at any token); the rows
+          // behind them are masked.
+          const int e = idx / n_spans;
+          sp = idx % n_spans;
+          const int i = far_sequence(p, e);
+          int s_p, e_p;
+          far_range(p, i, e - i, s_p, e_p, q_lo, q_hi);
+          t0 = max(s_p, p.span_pos[sp]);
+          n_valid_k = min(s_p + n_sink, p.span_pos[sp] + p.span_len[sp]) - t0;
+          key0 = t0 - p.span_pos[sp];
+          far = e + 1;
+          if (q_lo > q_hi || n_valid_k <= 0) {  // nothing: take the next item into the same slot
+            --n;
+            continue;
+          }
         } else {
-          pmax = (e_last - 1 - t_last > p.window) ? t_last + p.window : e_last - 1;
+          const int kt_g = kPlain ? idx : idx - p.far_segs * n_spans;
+          while (sp + 1 < n_spans && kt_g >= p.span_tile0[sp + 1]) ++sp;
+          key0 = (kt_g - p.span_tile0[sp]) * kTile;  // token offset inside the span
+          n_valid_k = min(kTile, p.span_len[sp] - key0);
+          t0 = p.span_pos[sp] + key0;
+          // query tiles that can see at least one key of this tile
+          const int t_last = t0 + n_valid_k - 1;
+          int s_last, e_last;
+          seq_of(cu_seq, n_seqs, t_last, s_last, e_last);
+          int pmax;
+          if (n_sink > 0 && p.far_segs == 0 && s_last + n_sink > t0) {
+            pmax = e_last - 1;  // the tile holds a sink token: every later query of that sequence
+          } else {
+            pmax = (e_last - 1 - t_last > p.window) ? t_last + p.window : e_last - 1;
+          }
+          q_lo = max(t0, p.q_pos_start);
+          q_hi = min(pmax, q_end_pos - 1);
         }
-        const int q_lo = max(t0, p.q_pos_start);
-        const int q_hi = min(pmax, q_end_pos - 1);
         int qt_first = 0, n_qt = 0;
         if (q_lo <= q_hi) {
           qt_first = (q_lo - p.q_pos_start) / kTile;
@@ -193,6 +216,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         }
         g->valid = 1, g->b = b, g->hk = hk, g->sp = sp, g->key0 = key0, g->n_valid_k = n_valid_k, g->t0 = t0;
         g->qt_first = qt_first, g->n_qt = n_qt;
+        g->far = far, g->far_hi = q_hi;
         mbar_arrive(&ctl->geom_full[slot]);
         if (n_qt == 0) continue;
         // K and V have one buffer each: the previous item's last S^T and dP^T products must have read them
@@ -358,6 +382,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
     bool pend = false;
     int pend_nk = 0, pend_sp = 0;
     long long pend_off = -1;  // element offset of this thread's 64 columns (-1: the key row does not exist)
+    float* pend_ws = nullptr;  // partial sums of a sink row (non-null: this row does not go to dk / dv)
     auto drain = [&]() -> bool {
       bool k = mbar_wait(&ctl->done, pend_nk & 1, err, kErrWaitEpilogue);
       k = __all_sync(0xffffffffu, k);
@@ -373,8 +398,8 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         const float mul = which == 0 ? p.scale : 1.f;
         void* base = which == 0 ? p.dk[pend_sp] : p.dv[pend_sp];
         if (pend_off < 0) continue;
-        if (f32) {
-          float* dst = static_cast<float*>(base) + pend_off + c * 32;
+        if (f32 || (!kPlain && pend_ws != nullptr)) {
+          float* dst = !kPlain && pend_ws != nullptr ? pend_ws + which * 128 + c * 32 : static_cast<float*>(base) + pend_off + c * 32;
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             uint32_t o[8];
@@ -413,13 +438,21 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
       const int n_iter = gm.n_qt * group;
       const bool valid_k = row < gm.n_valid_k;
       const int t = valid_k ? gm.t0 + row : 0x7fffffff;
-      int p_hi = -1;
+      // this key sees the queries [p_lo, p_hi]
+      int p_lo = t, p_hi = -1;
+      float* ws = nullptr;  // where this row's partial sums go instead of dk / dv
       if (valid_k) {
         int s_t, e_t;
-        seq_of(cu_seq, n_seqs, t, s_t, e_t);
+        const int i_t = seq_of(cu_seq, n_seqs, t, s_t, e_t);
         const bool is_sink = t < s_t + n_sink;
-        p_hi = (is_sink || e_t - 1 - t <= p.window) ? e_t - 1 : t + p.window;
+        const bool split = !kPlain && p.far_segs > 0;
+        p_hi = ((is_sink && !split) || e_t - 1 - t <= p.window) ? e_t - 1 : t + p.window;
         p_hi = min(p_hi, q_end_pos - 1);
+        if (split && is_sink && min(e_t, q_end_pos) - 1 - t > p.window) {
+          const int slot_ws = gm.far ? gm.far - 1 : p.far_segs + i_t;
+          ws = p.far_ws + ((static_cast<long long>(gm.b * p.hkv + gm.hk) * p.far_slots + slot_ws) * n_sink + (t - s_t)) * 256 + half * 64;
+        }
+        if (!kPlain && gm.far) p_lo = t + p.window + 1, p_hi = gm.far_hi;
       }
 
       int iq = 0;
@@ -429,7 +462,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         if (++iq == gm.n_qt) iq = 0;
         const float* lse_s = sLse + (g % kQStages) * kTile + half * 64;
         const float* del_s = sDelta + (g & 1) * kTile + half * 64;
-        const bool full = (pq0 >= t) && (pq0 + kTile - 1 <= p_hi);
+        const bool full = (pq0 >= p_lo) && (pq0 + kTile - 1 <= p_hi);
         const bool masked = !__all_sync(0xffffffffu, full);
 
         // P^T from S^T (the -lse2 row of this stage landed together with Q, before S^T was issued; the
@@ -443,14 +476,14 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
           // A tile the band edge or a sequence boundary crosses gets its hidden scores replaced by -inf
           // IN tensor memory, by a short rolled loop, and then takes the same code as every other tile
           // (the compares unrolled over the 64 columns inside the loop below were a tenth of the
-          // kernel, which has to fit the instruction cache).  This key sees the queries [t, p_hi].
-          const uint32_t qn = static_cast<uint32_t>(max(p_hi - t + 1, 0));
+          // kernel, which has to fit the instruction cache).
+          const uint32_t qn = static_cast<uint32_t>(max(p_hi - p_lo + 1, 0));
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
             uint32_t sm[32];
             tmem_ld32(tS + lane_off + half * 64 + c * 32, sm);
             tmem_ld_wait();
-            const int c0 = pq0 + half * 64 + c * 32 - t;
+            const int c0 = pq0 + half * 64 + c * 32 - p_lo;
 #pragma unroll
             for (int i = 0; i < 32; ++i) sm[i] = static_cast<uint32_t>(c0 + i) < qn ? sm[i] : 0xff800000u;
             tmem_st32(tS + lane_off + half * 64 + c * 32, sm);
@@ -560,20 +593,23 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         pend = true;
         pend_nk = nk;
         pend_sp = gm.sp;
-        pend_off = valid_k ? gm.b * p.dkv_sb[gm.sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[gm.sp] + gm.hk * p.dkv_sh[gm.sp] + half * 64 : -1;
+        pend_ws = ws;
+        // (a far item stores nothing for a row that has no far query: the row's key tile writes it directly)
+        pend_off = valid_k && (kPlain || gm.far == 0 || ws != nullptr) ? gm.b * p.dkv_sb[gm.sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[gm.sp] + gm.hk * p.dkv_sh[gm.sp] + half * 64 : -1;
         gbase += n_iter;
         ++nk;
       } else if (valid_k) {
         // no query of this call sees the tile: zero gradients
         const int sp = gm.sp;
         const long long off = gm.b * p.dkv_sb[sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[sp] + gm.hk * p.dkv_sh[sp] + half * 64;
-        const bool f32 = !kPlain && p.grad_fp32[sp] != 0;
+        const bool f32 = !kPlain && (p.grad_fp32[sp] != 0 || ws != nullptr);
         const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll 1
         for (int which = 0; which < 2; ++which) {
           void* base = which == 0 ? p.dk[sp] : p.dv[sp];
           const int n32 = f32 ? 8 : 4;  // 32-byte pieces of this thread's 64 columns
           uint8_t* dst = f32 ? reinterpret_cast<uint8_t*>(static_cast<float*>(base) + off) : reinterpret_cast<uint8_t*>(static_cast<uint16_t*>(base) + off);
+          if (!kPlain && ws != nullptr) dst = reinterpret_cast<uint8_t*>(ws + which * 128);
 #pragma unroll 1
           for (int v = 0; v < n32; ++v) st_global_v8(dst + v * 32, z);
         }
@@ -592,10 +628,45 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
   if (threadIdx.x == 0 && ctl->err != 0) atomicCAS(p.status, 0, ctl->err);
 }
 
+// Adds up the parts of the sink rows' gradients: the windowed part and the far segments of the row's sequence,
+// in a fixed order.  One block per (batch row, KV head, sequence, sink row); thread = (dK or dV, column).
+// A handful of 512-byte rows per block: latency, 4 us where it replaced a serial chain of milliseconds.
+template <bool kBf16>
+__global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ BwdKernelParams p) {
+  const int r = blockIdx.x % p.n_sink, i = blockIdx.x / p.n_sink;
+  const int hk = blockIdx.y, b = blockIdx.z;
+  int s, e, q_lo, q_hi;
+  far_range(p, i, 0, s, e, q_lo, q_hi);
+  const int t = s + r;
+  if (t >= e || min(e, p.q_pos_start + p.q_len) - 1 - t <= p.window) return;  // no far query: dk / dv hold the result
+  int sp = 0;
+  while (sp < p.n_spans && (t < p.span_pos[sp] || t >= p.span_pos[sp] + p.span_len[sp])) ++sp;
+  if (sp == p.n_spans) return;
+  const float* ws = p.far_ws + (static_cast<long long>(b * p.hkv + hk) * p.far_slots * p.n_sink + r) * 256 + threadIdx.x;
+  const long long slot = p.n_sink * 256LL;
+  float sum = ws[(p.far_segs + i) * slot];
+  // chunk boundaries below the sequence's start / its end (a start comes first on a tie): the segments are
+  // i + j for j in between
+  const int n_b = (p.q_len + p.far_chunk - 1) / p.far_chunk - 1;
+  auto below = [&](int x) { return x <= p.q_pos_start ? 0 : min(n_b, (x - p.q_pos_start - 1) / p.far_chunk); };
+  const int j1 = below(e);
+#pragma unroll 4
+  for (int j = p.cu == nullptr ? 0 : below(s); j <= j1; ++j) {
+    far_range(p, i, j, s, e, q_lo, q_hi);
+    if (q_lo <= q_hi) sum += ws[(i + j) * slot];
+  }
+  const int which = threadIdx.x >> 7, c = threadIdx.x & 127;
+  const long long off = b * p.dkv_sb[sp] + static_cast<long long>(t - p.span_pos[sp]) * p.dkv_st[sp] + hk * p.dkv_sh[sp] + c;
+  void* base = which == 0 ? p.dk[sp] : p.dv[sp];
+  if (p.grad_fp32[sp]) static_cast<float*>(base)[off] = sum;
+  else static_cast<uint16_t*>(base)[off] = static_cast<uint16_t>(pack2<kBf16>(sum, 0.f));
+}
+
 }  // namespace
 
 int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaStream_t stream) {
-  const long long n_cta = static_cast<long long>(total_key_tiles) * kp.hkv * kp.batch;
+  // far items (see BwdKernelParams) come first: they are the longest where the segments' sequences are long
+  const long long n_cta = (static_cast<long long>(total_key_tiles) + static_cast<long long>(kp.far_segs) * kp.n_spans) * kp.hkv * kp.batch;
   if (n_cta <= 0) return RSWA_OK;
   if (n_cta > 0x7fffffffLL) {
     set_error("rswa_bwd: too many key tiles (%lld)", n_cta);
@@ -626,6 +697,17 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaSt
   if (e != cudaSuccess) {
     set_error("rswa_bwd: launch: %s", cudaGetErrorString(e));
     return RSWA_E_CUDA;
+  }
+  if (kp.far_segs > 0) {
+    const int n_seq = kp.cu == nullptr ? 1 : kp.n_seqs + 1;
+    const dim3 grid(static_cast<unsigned>(n_seq * kp.n_sink), static_cast<unsigned>(kp.hkv), static_cast<unsigned>(kp.batch));
+    if (dtype == RSWA_DTYPE_BF16) sink_sum_kernel<true><<<grid, 256, 0, stream>>>(kp);
+    else sink_sum_kernel<false><<<grid, 256, 0, stream>>>(kp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) {
+      set_error("rswa_bwd: sink sums: launch: %s", cudaGetErrorString(e));
+      return RSWA_E_CUDA;
+    }
   }
   return RSWA_OK;
 }

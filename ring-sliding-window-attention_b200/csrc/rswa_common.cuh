@@ -73,15 +73,23 @@ struct BwdKernelParams {
   int* dkv_counter;  // work counter of the dK/dV kernel, likewise
   long long dq_sb, dq_st, dq_sh;
   int* status;
+  // Sink tokens are seen by every later query of their sequence.  When far_segs > 0 the dK/dV kernel treats
+  // the queries beyond a sink token's window separately: the query axis is cut into far_segs segments
+  // (see far_segment), each a work item of its own per KV head, whose dK / dV of the sink rows go to far_ws
+  // as partial sums ([batch, hkv, far_segs + sequences, n_sink, 2, 128] fp32; the rows' windowed part goes to
+  // the slot far_segs + sequence) and are added up by sink_sum_kernel.
+  int far_segs, far_chunk, far_slots;  // far_chunk: positions per chunk, a multiple of the tile
+  float* far_ws;
 };
 
 // Sequence [start, end) containing global position p.  cu has n_seqs + 1 entries.
-__device__ __forceinline__ void seq_of(const int* __restrict__ cu, int n_seqs, int p, int& start,
-                                       int& end) {
+// Returns its index (tokens past the last boundary form a sequence of their own, index n_seqs).
+__device__ __forceinline__ int seq_of(const int* __restrict__ cu, int n_seqs, int p, int& start,
+                                      int& end) {
   if (cu == nullptr) {
     start = 0;
     end = 0x7fffffff;
-    return;
+    return 0;
   }
   int lo = 0, hi = n_seqs;
   while (lo < hi) {
@@ -90,6 +98,36 @@ __device__ __forceinline__ void seq_of(const int* __restrict__ cu, int n_seqs, i
   }
   start = __ldg(cu + lo);
   end = (lo < n_seqs) ? __ldg(cu + lo + 1) : 0x7fffffff;
+  return lo;
+}
+
+// The query axis of a call, cut at multiples of far_chunk from its first query and at sequence starts:
+// segment e lies in one sequence and one chunk.  With i sequence starts and j chunk boundaries in front of
+// it, e = i + j and it belongs to sequence i.  Fills the sequence's bounds and the positions [q_lo, q_hi] of the
+// segment's queries that lie beyond the window of the sequence's first token (none if q_lo > q_hi).
+__device__ __forceinline__ void far_range(const BwdKernelParams& p, int i, int j, int& s, int& e, int& q_lo, int& q_hi) {
+  s = 0, e = 0x7fffffff;
+  if (p.cu != nullptr) {
+    s = __ldg(p.cu + i);
+    if (i < p.n_seqs) e = __ldg(p.cu + i + 1);
+  }
+  const int q_end = p.q_pos_start + p.q_len;
+  const int n_chunks = (p.q_len + p.far_chunk - 1) / p.far_chunk;
+  const int a = p.q_pos_start + j * p.far_chunk;
+  const int z = j + 1 < n_chunks ? a + p.far_chunk : q_end;
+  q_lo = max(max(s, a), s > 0x7ffffffe - p.window ? 0x7fffffff : s + p.window + 1);
+  q_hi = min(e, z) - 1;
+}
+// number of sequence starts among the first e of the merged boundaries (starts first on ties)
+__device__ __forceinline__ int far_sequence(const BwdKernelParams& p, int e) {
+  if (p.cu == nullptr) return 0;
+  const int n_b = (p.q_len + p.far_chunk - 1) / p.far_chunk - 1;  // boundary j at q_pos_start + (j + 1) * far_chunk
+  int lo = max(0, e - n_b), hi = min(e, p.n_seqs);                // start i at cu[i + 1]
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(p.cu + mid + 1) <= p.q_pos_start + (e - mid) * p.far_chunk) lo = mid + 1; else hi = mid;
+  }
+  return lo;
 }
 
 // Optional in-kernel timeline (development builds only, -DRSWA_TRACE): one chosen CTA stamps clock64()

@@ -235,11 +235,15 @@ def fwd(q: torch.Tensor, spans: Sequence[KVSpan], window: int, n_sink: int, scal
     return out, lse
 
 
-def bwd_workspace(q: torch.Tensor) -> torch.Tensor:
+def bwd_workspace(q: torch.Tensor, n_kv_heads: int = 0, window: int = 0, n_sink: int = 0, n_seqs: int = 0) -> torch.Tensor:
+    """Scratch of a backward over q; with the arguments of a call with sink tokens also the partial sums
+    that let their gradients be computed in parallel."""
     B, S, Hq, D = q.shape
     n = _C.lib().rswa_bwd_workspace_bytes(B, S, Hq, D)
     if n < 0:
         raise ValueError("rswa_bwd_workspace_bytes: unsupported shape")
+    if n_sink > 0:
+        n += _C.lib().rswa_bwd_sink_workspace_bytes(B, S, n_kv_heads, window, n_sink, n_seqs)
     return torch.empty(n, dtype=torch.uint8, device=q.device)
 
 
@@ -257,7 +261,8 @@ def bwd(q: torch.Tensor, spans: Sequence[KVSpan], out: torch.Tensor, lse: torch.
         if t.dtype != q.dtype or t.shape != q.shape:
             raise ValueError(f"{name} must match q in dtype and shape")
     if workspace is None:
-        workspace = bwd_workspace(q)
+        workspace = bwd_workspace(q, spans[0].k.shape[2] if spans else q.shape[2], window, n_sink,
+                                  0 if cu_seqlens is None else cu_seqlens.numel() - 1)
     p = _C.BwdParams()
     _fill_geom(p.g, q, spans, window, n_sink, scale, q_pos_start, cu_seqlens, grads=True)
     p.q = q.data_ptr()

@@ -279,7 +279,10 @@ class RingAttn(torch.autograd.Function):
         remote = sink_remote + remote
 
         dq4 = torch.empty_like(q4)
-        ws = K.bwd_workspace(q4)
+        if args["n_sink"] and q4.is_cuda:
+            ws = K.bwd_workspace(q4, k4.shape[2], args["window"], args["n_sink"], 0 if cu_seqlens is None else cu_seqlens.numel() - 1)
+        else:
+            ws = K.bwd_workspace(q4)
         link = ctx.link
         ops, recvs = [], []   # recvs: (offset, tokens, gradient tensor, (hop, sender) when it sits in a peer slot)
         # With peer stores (a copy-engine put behind an event, no message that the host must post between

@@ -166,6 +166,28 @@ def test_spans_emulated_ranks(cp, S, W, n_sink, lens):
     assert_close("dv", dv_acc, rdv)
 
 
+# The queries beyond a sink token's window are cut into segments of 4 query tiles (window below 256 tokens) at
+# sequence starts, where the axis has at least twice as many tiles as a key's window.
+@pytest.mark.parametrize("B,S,W,n_sink,lens", [
+    (1, 512, 60, 1, None),                        # one segment: the smallest axis that is cut
+    (2, 1030, 60, 2, None),                       # three segments, the last of six tokens
+    (1, 1400, 300, 16, None),                     # the most sink tokens that are kept as partial sums
+    (1, 1400, 100, 17, None),                     # ... one more: not cut
+    # sequences start on, before and behind a cut.  (A window of 0 would leave each sink token a quarter of
+    # every query's weight: 2148 terms of ~1 rounded to 16 bits add up to sqrt(2148) * 2^-9 = 0.09, above the
+    # fixed bound of 2e-2; with 24 keys the terms are a sixth of that.)
+    (1, 2100, 20, 3, [512, 511, 1, 2, 1074]),
+])
+def test_sink_gradients_in_segments(B, S, W, n_sink, lens):
+    test_fwd_bwd_matches_oracle("segments", B, S, 4, 2, W, n_sink, lens)
+
+
+@pytest.mark.parametrize("cp,S,lens", [(2, 1100, [1098, 1102]), (2, 1152, [2304])])
+def test_sink_gradients_in_segments_over_spans(cp, S, lens):
+    """Sink tokens on two spans of a call, and queries that start behind the sink tokens' rank."""
+    test_spans_emulated_ranks(cp, S, 70, 4, lens)
+
+
 def test_two_phase_forward_and_split_backward():
     """Query-tile ranges, the (local | halo) partials + merge path and a backward split over two calls."""
     from ring_swa import _C
