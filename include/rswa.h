@@ -273,6 +273,14 @@ int rswa_event_wait(void* ev, void* stream);
 /* milliseconds between two recorded events, after synchronising on `stop`; negative on error */
 float rswa_event_elapsed_ms(void* start, void* stop);
 
+/* Kernels of this library launched by the process so far. */
+int64_t rswa_launch_count(void);
+
+/* Names a host-visible word (mapped pinned memory) into which every kernel given `status` also writes the code
+ * it raises or finds raised there: the host then learns of a time-out by reading its own memory, with no copy
+ * or synchronisation on the stream.  mirror NULL takes it back. */
+int rswa_set_status_mirror(const int32_t* status, int32_t* mirror);
+
 int rswa_abi_version(void);
 const char* rswa_last_error(void);
 

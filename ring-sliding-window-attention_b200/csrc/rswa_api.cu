@@ -1,7 +1,9 @@
 // C-ABI layer: argument checks, TMA descriptor set-up, launches.  See include/rswa.h.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "rswa_common.cuh"
 
@@ -9,7 +11,7 @@ namespace rswa {
 
 int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream);
 int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaStream_t stream);
-int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, cudaStream_t stream);
+int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, int* counters, cudaStream_t stream);
 int launch_dq(const BwdKernelParams& kp, int dtype, cudaStream_t stream);
 
 static thread_local char g_err[512] = "";
@@ -19,6 +21,29 @@ void set_error(const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_err, sizeof(g_err), fmt, ap);
   va_end(ap);
+}
+
+static std::atomic<long long> g_launches{0};
+void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+// Status words and their host-visible mirrors: a handful per process (one per device), entries are added under
+// the lock and read without it.
+namespace {
+struct MirrorEntry {
+  std::atomic<const int*> status{nullptr};
+  std::atomic<int*> mirror{nullptr};
+};
+constexpr int kMaxMirrors = 64;
+MirrorEntry g_mirror[kMaxMirrors];
+std::atomic<int> g_n_mirrors{0};
+std::mutex g_mirror_mutex;
+}  // namespace
+
+int* status_mirror(const int* status) {
+  const int n = g_n_mirrors.load(std::memory_order_acquire);
+  for (int i = 0; i < n; ++i)
+    if (g_mirror[i].status.load(std::memory_order_relaxed) == status) return g_mirror[i].mirror.load(std::memory_order_relaxed);
+  return nullptr;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -234,6 +259,22 @@ using namespace rswa;
 
 extern "C" int rswa_abi_version(void) { return RSWA_ABI_VERSION; }
 extern "C" const char* rswa_last_error(void) { return g_err; }
+extern "C" int64_t rswa_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+
+extern "C" int rswa_set_status_mirror(const int32_t* status, int32_t* mirror) {
+  std::lock_guard<std::mutex> lock(g_mirror_mutex);
+  const int n = g_n_mirrors.load(std::memory_order_relaxed);
+  int i = 0;
+  while (i < n && g_mirror[i].status.load(std::memory_order_relaxed) != status) ++i;
+  if (status == nullptr || i == kMaxMirrors) {
+    set_error("rswa_set_status_mirror: null status word, or more than %d of them", kMaxMirrors);
+    return RSWA_E_ARG;
+  }
+  g_mirror[i].status.store(status, std::memory_order_relaxed);
+  g_mirror[i].mirror.store(mirror, std::memory_order_relaxed);
+  if (i == n) g_n_mirrors.store(n + 1, std::memory_order_release);
+  return RSWA_OK;
+}
 
 extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
   if (p == nullptr) {
@@ -286,6 +327,7 @@ extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
   kp.n_q_tiles = qe - qb;
   kp.carry = p->carry != 0;
   kp.status = p->status;
+  kp.mirror = status_mirror(p->status);
   return launch_fwd(kp, g.dtype, static_cast<cudaStream_t>(stream));
 }
 
@@ -336,7 +378,7 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   float* delta = static_cast<float*>(p->workspace);
   float* lse2 = delta + static_cast<int64_t>(g.batch) * g.n_q_heads * q_len_pad;
   int* dq_counter = reinterpret_cast<int*>(lse2 + static_cast<int64_t>(g.batch) * g.n_q_heads * q_len_pad);
-  {  // both work counters, ahead of every kernel of this call, so that the reset sits in no timed interval
+  if (!(p->flags & RSWA_BWD_INIT)) {  // both work counters; with INIT the delta kernel resets them
     cudaError_t e = cudaMemsetAsync(dq_counter, 0, 2 * sizeof(int), static_cast<cudaStream_t>(stream_));
     if (e != cudaSuccess) {
       set_error("rswa_bwd: cudaMemsetAsync: %s", cudaGetErrorString(e));
@@ -376,6 +418,7 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   kq.dq_st = p->dq_stride_t;
   kq.dq_sh = p->dq_stride_h;
   kq.status = p->status;
+  kq.mirror = status_mirror(p->status);
 
   kk = kq;
   int n_k = 0, total_tiles = 0;
@@ -417,7 +460,7 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   }
 
   if (p->flags & RSWA_BWD_INIT) {
-    rc = launch_delta(*p, delta, lse2, q_len_pad, stream);
+    rc = launch_delta(*p, delta, lse2, q_len_pad, dq_counter, stream);
     if (rc) return rc;
   }
   if (p->ev_main_start) cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream);

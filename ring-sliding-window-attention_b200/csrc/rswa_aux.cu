@@ -40,7 +40,9 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
                              const uint16_t* __restrict__ dout, long long d_sb, long long d_st, long long d_sh,
                              const float* __restrict__ lse, long long l_sb, long long l_sh,
                              float* __restrict__ delta, float* __restrict__ lse2, int batch, int q_len, int hq,
-                             int q_len_pad) {
+                             int q_len_pad, int* __restrict__ counters) {
+  // the work counters of the two kernels behind this one (a memset of 8 bytes would be a launch of its own)
+  if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // warp task
   const int lane = threadIdx.x & 31;
   const int sub = lane & 15, hi = lane >> 4;
@@ -314,6 +316,7 @@ __global__ void cast_kernel(uint16_t* __restrict__ dst, long long dst_sb, const 
 }
 
 int check_launch(const char* what) {
+  count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("%s: launch: %s", what, cudaGetErrorString(e));
@@ -324,7 +327,7 @@ int check_launch(const char* what) {
 
 }  // namespace
 
-int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, cudaStream_t stream) {
+int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, int* counters, cudaStream_t stream) {
   const rswa_geom_t& g = p.g;
   const long long tasks = static_cast<long long>(g.batch) * g.n_q_heads * (q_len_pad / 32);  // one warp each
   const int threads = 256;
@@ -333,7 +336,7 @@ int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_le
   kern<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
       static_cast<const uint16_t*>(p.out), p.o_stride_b, p.o_stride_t, p.o_stride_h,
       static_cast<const uint16_t*>(p.dout), p.do_stride_b, p.do_stride_t, p.do_stride_h, p.lse, p.lse_stride_b,
-      p.lse_stride_h, delta, lse2, g.batch, g.q_len, g.n_q_heads, q_len_pad);
+      p.lse_stride_h, delta, lse2, g.batch, g.q_len, g.n_q_heads, q_len_pad, counters);
   return check_launch("rswa_bwd(delta)");
 }
 

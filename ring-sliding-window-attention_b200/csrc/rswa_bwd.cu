@@ -101,8 +101,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
   float* sDelta = sLse + kQStages * kTile;                       // [2][128], travels with dO
   BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + kBwdSmemTiles + (kQStages + 2) * kRowBytes);
 
-  // a device-side error was already reported on this stream: do not pile further time-outs on it
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(p.status) != 0)) return;
+  if (status_raised(p.status, p.mirror)) return;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -625,7 +624,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
     tc_fence_after();
     tmem_dealloc(tmem, kBwdTmemCols);
   }
-  if (threadIdx.x == 0 && ctl->err != 0) atomicCAS(p.status, 0, ctl->err);
+  if (threadIdx.x == 0 && ctl->err != 0) raise_status(p.status, p.mirror, ctl->err);
 }
 
 // Adds up the parts of the sink rows' gradients: the windowed part and the far segments of the row's sequence,
@@ -693,6 +692,7 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaSt
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_grid = n_cta < sm_count() ? n_cta : sm_count();
   kern<<<static_cast<unsigned>(n_grid), kBwdThreads, kBwdSmemBytes, stream>>>(kp, static_cast<int>(n_cta));
+  count_launches(kp.far_segs > 0 ? 2 : 1);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rswa_bwd: launch: %s", cudaGetErrorString(e));

@@ -41,6 +41,7 @@ struct FwdKernelParams {
   int q_tile_begin, n_q_tiles;
   int carry;  // out / lse hold a partial result over other keys: continue it instead of starting over
   int* status;
+  int* mirror;  // host-visible copy of the status word (or null)
 };
 
 struct BwdKernelParams {
@@ -73,6 +74,7 @@ struct BwdKernelParams {
   int* dkv_counter;  // work counter of the dK/dV kernel, likewise
   long long dq_sb, dq_st, dq_sh;
   int* status;
+  int* mirror;  // host-visible copy of the status word (or null)
   // Sink tokens are seen by every later query of their sequence.  When far_segs > 0 the dK/dV kernel treats
   // the queries beyond a sink token's window separately: the query axis is cut into far_segs segments
   // (see far_segment), each a work item of its own per KV head, whose dK / dV of the sink rows go to far_ws
@@ -81,6 +83,20 @@ struct BwdKernelParams {
   int far_segs, far_chunk, far_slots;  // far_chunk: positions per chunk, a multiple of the tile
   float* far_ws;
 };
+
+// True in every thread of the block if an error was already reported through the status word: the kernel then
+// does no work, so as not to pile further time-outs on it.  The report also goes to the host-visible mirror,
+// from where the host picks it up without a copy or a synchronisation.
+__device__ __forceinline__ bool status_raised(const int* status, int* mirror) {
+  const int code = *reinterpret_cast<const volatile int*>(status);
+  if (!__syncthreads_or(code != 0)) return false;
+  if (mirror != nullptr && threadIdx.x == 0 && code != 0) *reinterpret_cast<volatile int*>(mirror) = code;
+  return true;
+}
+__device__ __forceinline__ void raise_status(int* status, int* mirror, int code) {
+  atomicCAS(status, 0, code);
+  if (mirror != nullptr) *reinterpret_cast<volatile int*>(mirror) = code;
+}
 
 // Sequence [start, end) containing global position p.  cu has n_seqs + 1 entries.
 // Returns its index (tokens past the last boundary form a sequence of their own, index n_seqs).
@@ -158,6 +174,8 @@ void set_error(const char* fmt, ...);
 int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int tokens, int heads,
                   long long sb, long long st, long long sh);
 int check_geom(const rswa_geom_t& g, bool need_grads);
+int* status_mirror(const int* status);  // the mirror registered for a status word, or null
+void count_launches(int n);             // kernels of this library launched (rswa_launch_count)
 int sm_count();  // SMs of the current device (cached per device)
 
 }  // namespace rswa

@@ -100,8 +100,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
   uint8_t* sV = smem + 5 * kTileBytes;  // two stages
   DqCtl* ctl = reinterpret_cast<DqCtl*>(smem + kDqSmemTiles);
 
-  // a device-side error was already reported on this stream: do not pile further time-outs on it
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(p.status) != 0)) return;
+  if (status_raised(p.status, p.mirror)) return;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -539,7 +538,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
     tc_fence_after();
     tmem_dealloc(tmem, kDqTmemCols);
   }
-  if (threadIdx.x == 0 && ctl->err != 0) atomicCAS(p.status, 0, ctl->err);
+  if (threadIdx.x == 0 && ctl->err != 0) raise_status(p.status, p.mirror, ctl->err);
 }
 
 }  // namespace
@@ -573,6 +572,7 @@ int launch_dq(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_cta = n_items < sm_count() ? n_items : sm_count();
   kern<<<static_cast<unsigned>(n_cta), kDqThreads, kDqSmemBytes, stream>>>(kp, n_q_tiles, static_cast<int>(n_items));
+  count_launches(1);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rswa_bwd(dq): launch: %s", cudaGetErrorString(e));

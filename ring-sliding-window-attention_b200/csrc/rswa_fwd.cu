@@ -124,8 +124,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
   FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + kFwdSmemTiles);
 
   RSWA_TRC(fwd, threadIdx.x == 0, 1920);
-  // a device-side error was already reported on this stream: do not pile further time-outs on it
-  if (__syncthreads_or(*reinterpret_cast<volatile int*>(p.status) != 0)) return;
+  if (status_raised(p.status, p.mirror)) return;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -641,7 +640,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
     tmem_dealloc(tmem, kFwdTmemCols);
   }
   RSWA_TRC(fwd, threadIdx.x == 32, 1923);
-  if (threadIdx.x == 0 && ctl->err != 0) atomicCAS(p.status, 0, ctl->err);
+  if (threadIdx.x == 0 && ctl->err != 0) raise_status(p.status, p.mirror, ctl->err);
 }
 
 }  // namespace
@@ -677,6 +676,7 @@ int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream) {
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_cta = n_items < sm_count() ? n_items : sm_count();
   kern<<<static_cast<unsigned>(n_cta), kFwdThreads, kFwdSmemBytes, stream>>>(kp, n_blocks, static_cast<int>(n_items));
+  count_launches(1);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rswa_fwd: launch: %s", cudaGetErrorString(e));

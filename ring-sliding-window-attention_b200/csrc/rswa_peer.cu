@@ -30,8 +30,8 @@ __global__ void flag_set_kernel(int* flag, int value) {
   asm volatile("st.release.sys.global.b32 [%0], %1;" ::"l"(flag), "r"(value) : "memory");
 }
 
-__global__ void flag_wait_kernel(const int* flag, int value, int* status, unsigned long long timeout_ns) {
-  if (*reinterpret_cast<volatile int*>(status) != 0) return;  // an error was already reported on this stream
+__global__ void flag_wait_kernel(const int* flag, int value, int* status, int* mirror, unsigned long long timeout_ns) {
+  if (status_raised(status, mirror)) return;
   unsigned long long t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   for (;;) {
@@ -43,10 +43,11 @@ __global__ void flag_wait_kernel(const int* flag, int value, int* status, unsign
     if (now - t0 > timeout_ns) break;
     __nanosleep(200);
   }
-  atomicCAS(status, 0, kErrWaitFlag);
+  raise_status(status, mirror, kErrWaitFlag);
 }
 
 int check_launch_peer(const char* what) {
+  count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("%s: %s", what, cudaGetErrorString(e));
@@ -95,7 +96,7 @@ extern "C" int rswa_flag_wait(const int32_t* flag, int32_t value, int32_t* statu
     set_error("rswa_flag_wait: flag, status and a positive time limit are required");
     return RSWA_E_ARG;
   }
-  flag_wait_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(flag, value, status,
+  flag_wait_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(flag, value, status, status_mirror(status),
                                                                   static_cast<unsigned long long>(timeout_ns));
   return check_launch_peer("rswa_flag_wait");
 }

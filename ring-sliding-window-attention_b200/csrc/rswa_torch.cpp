@@ -1,0 +1,256 @@
+// The single-GPU call of the public functions, host side in C++: one autograd function that allocates the
+// results, fills the C ABI's parameter structs and launches.
+//
+// A training step on a few thousand tokens takes the GPU 40-300 us; through Python and ctypes (the ring's path,
+// ring_swa/_ring.py) its two calls took the host 340 us -- the interpreter in the autograd engine's thread, a
+// field-by-field ctypes struct, torch's Python tensor constructors -- and the GPU waited.  Here a forward call
+// takes the host about 10 us and a backward 15.
+//
+// attention() returns None whenever a call is not an ordinary one (other dtypes or devices, an error to report,
+// no status word yet): the Python path then runs it, or raises what it raises.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cmath>
+#include <cstring>
+
+#include "../../include/rswa.h"
+
+namespace {
+
+constexpr int kMaxDevices = 64;
+constexpr int64_t kMaxHeadDim = 128;
+// per device: the status word the kernels raise and its host mirror (ring_swa/_kernels.py owns both)
+int32_t* g_status[kMaxDevices] = {nullptr};
+const volatile int32_t* g_mirror[kMaxDevices] = {nullptr};
+
+// [tokens, heads, D] (packed sequences) or [batch, tokens, heads, D]
+struct Dims {
+  int64_t batch, tokens, heads;
+};
+Dims dims_of(const at::Tensor& t) {
+  if (t.dim() == 3) return {1, t.size(0), t.size(1)};
+  return {t.size(0), t.size(1), t.size(2)};
+}
+struct Strides {
+  int64_t b, t, h;
+};
+Strides strides_of(const at::Tensor& t) {
+  if (t.dim() == 3) return {0, t.stride(0), t.stride(1)};
+  return {t.stride(0), t.stride(1), t.stride(2)};
+}
+
+// The kernels address tensors through TMA descriptors: positive strides in multiples of 16 bytes, the head
+// dimension contiguous.  Anything else (expanded gradients, odd slices) is copied.
+bool dense_enough(const at::Tensor& t) {
+  const auto st = t.strides();
+  if (st.back() != 1 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0) return false;
+  for (size_t i = 0; i + 1 < st.size(); ++i)
+    if (st[i] <= 0 || st[i] % 8 != 0) return false;
+  return true;
+}
+at::Tensor dense(const at::Tensor& t) { return dense_enough(t) ? t : t.contiguous(); }
+
+struct Call {
+  int64_t window, n_sink;
+  double scale;
+};
+
+void fill_geom(rswa_geom_t& g, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu, const Call& c) {
+  const Dims dq = dims_of(q), dk = dims_of(k);
+  const Strides sk = strides_of(k);
+  g.dtype = q.scalar_type() == at::kBFloat16 ? RSWA_DTYPE_BF16 : RSWA_DTYPE_FP16;
+  g.batch = static_cast<int32_t>(dq.batch);
+  g.q_len = static_cast<int32_t>(dq.tokens);
+  g.n_q_heads = static_cast<int32_t>(dq.heads);
+  g.n_kv_heads = static_cast<int32_t>(dk.heads);
+  g.head_dim = static_cast<int32_t>(q.size(-1));
+  g.window = static_cast<int32_t>(c.window);
+  g.n_sink = static_cast<int32_t>(c.n_sink);
+  g.softmax_scale = static_cast<float>(c.scale);
+  if (cu.defined()) {
+    g.cu_seqlens = cu.const_data_ptr<int32_t>();
+    g.n_seqs = static_cast<int32_t>(cu.numel() - 1);
+  }
+  g.n_spans = 1;
+  rswa_span_t& s = g.spans[0];
+  s.k = k.data_ptr();
+  s.v = v.data_ptr();
+  s.kv_stride_b = sk.b, s.kv_stride_t = sk.t, s.kv_stride_h = sk.h;
+  s.len = static_cast<int32_t>(dk.tokens);
+}
+
+void check(int rc, const char* what) {
+  if (rc == RSWA_OK) return;
+  if (rc == RSWA_E_ARG || rc == RSWA_E_UNSUPPORTED) TORCH_CHECK_VALUE(false, what, ": ", rswa_last_error());
+  TORCH_CHECK(false, what, ": ", rswa_last_error(), " (code ", rc, ")");
+}
+
+at::Tensor forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu, const Call& c, at::Tensor& lse) {
+  const Dims d = dims_of(q);
+  at::Tensor out = at::empty_like(q);
+  lse = at::empty({d.batch, d.heads, d.tokens}, q.options().dtype(at::kFloat));
+  rswa_fwd_params_t p;
+  std::memset(&p, 0, sizeof(p));
+  fill_geom(p.g, q, k, v, cu, c);
+  const Strides sq = strides_of(q), so = strides_of(out);
+  p.q = q.data_ptr();
+  p.q_stride_b = sq.b, p.q_stride_t = sq.t, p.q_stride_h = sq.h;
+  p.out = out.data_ptr();
+  p.o_stride_b = so.b, p.o_stride_t = so.t, p.o_stride_h = so.h;
+  p.lse = lse.data_ptr<float>();
+  p.lse_stride_b = d.heads * d.tokens, p.lse_stride_h = d.tokens;
+  p.status = g_status[q.get_device()];
+  check(rswa_fwd(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_fwd");
+  return out;
+}
+
+class SwaFunction : public torch::autograd::Function<SwaFunction> {
+ public:
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                            const std::optional<at::Tensor>& cu_, int64_t window, int64_t n_sink, double scale) {
+    const at::Tensor cu = cu_.has_value() ? *cu_ : at::Tensor();
+    at::Tensor lse;
+    at::Tensor out = ::forward(q, k, v, cu, {window, n_sink, scale}, lse);
+    ctx->save_for_backward({q, k, v, out, lse, cu});
+    ctx->saved_data["window"] = window;
+    ctx->saved_data["n_sink"] = n_sink;
+    ctx->saved_data["scale"] = scale;
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4], &cu = saved[5];
+    const Call c = {ctx->saved_data["window"].toInt(), ctx->saved_data["n_sink"].toInt(), ctx->saved_data["scale"].toDouble()};
+    const c10::cuda::CUDAGuard guard(q.device());
+    const at::Tensor dout = dense(grads[0]);
+    at::Tensor dq = at::empty_like(q);
+    at::Tensor dk = at::empty(k.sizes(), k.options()), dv = at::empty(k.sizes(), k.options());
+    const Dims d = dims_of(q);
+    const int64_t hkv = dims_of(k).heads;
+    int64_t ws_bytes = rswa_bwd_workspace_bytes(d.batch, d.tokens, d.heads, q.size(-1));
+    if (c.n_sink > 0) ws_bytes += rswa_bwd_sink_workspace_bytes(d.batch, d.tokens, hkv, c.window, c.n_sink, cu.defined() ? cu.numel() - 1 : 0);
+    at::Tensor ws = at::empty({ws_bytes}, q.options().dtype(at::kByte));
+
+    rswa_bwd_params_t p;
+    std::memset(&p, 0, sizeof(p));
+    fill_geom(p.g, q, k, v, cu, c);
+    rswa_span_t& s = p.g.spans[0];
+    const Strides skv = strides_of(dk);
+    s.dk = dk.data_ptr();
+    s.dv = dv.data_ptr();
+    s.dkv_stride_b = skv.b, s.dkv_stride_t = skv.t, s.dkv_stride_h = skv.h;
+    const Strides sq = strides_of(q), so = strides_of(out), sd = strides_of(dout), sdq = strides_of(dq);
+    p.q = q.data_ptr();
+    p.q_stride_b = sq.b, p.q_stride_t = sq.t, p.q_stride_h = sq.h;
+    p.out = out.data_ptr();
+    p.o_stride_b = so.b, p.o_stride_t = so.t, p.o_stride_h = so.h;
+    p.dout = dout.data_ptr();
+    p.do_stride_b = sd.b, p.do_stride_t = sd.t, p.do_stride_h = sd.h;
+    p.lse = lse.data_ptr<float>();
+    p.lse_stride_b = d.heads * d.tokens, p.lse_stride_h = d.tokens;
+    p.dq = dq.data_ptr();
+    p.dq_stride_b = sdq.b, p.dq_stride_t = sdq.t, p.dq_stride_h = sdq.h;
+    p.workspace = ws.data_ptr();
+    p.workspace_bytes = ws_bytes;
+    p.flags = RSWA_BWD_INIT | RSWA_BWD_FINISH;
+    p.status = g_status[q.get_device()];
+    check(rswa_bwd(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_bwd");
+    return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+};
+
+bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu) {
+  if (!q.is_cuda() || q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
+  if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf) return false;
+  if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;
+  if (k.device() != q.device() || v.device() != q.device()) return false;
+  const int dev = q.get_device();
+  if (dev < 0 || dev >= kMaxDevices || g_mirror[dev] == nullptr || *g_mirror[dev] != 0) return false;
+  if (dev != c10::cuda::current_device()) return false;
+  if (q.dim() != (cu.defined() ? 3 : 4) || k.dim() != q.dim() || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return false;
+  if (q.size(-1) != kMaxHeadDim || k.size(-1) != kMaxHeadDim) return false;
+  const Dims dq = dims_of(q), dk = dims_of(k);
+  if (dq.batch != dk.batch || dq.tokens != dk.tokens || dq.heads % dk.heads != 0) return false;
+  if (dq.batch > 0x7fffffff || dq.tokens > 0x7fffffff || dq.heads > 0x7fffffff) return false;
+  if (cu.defined() && (!cu.is_cuda() || cu.get_device() != dev || cu.scalar_type() != at::kInt || cu.dim() != 1 || !cu.is_contiguous() || cu.numel() < 2))
+    return false;
+  return true;
+}
+
+// attention(q, k, v, window, n_sink, scale or None, cu_seqlens or None) -> out, or None (see above)
+PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 7) {
+    PyErr_SetString(PyExc_TypeError, "attention takes 7 arguments");
+    return nullptr;
+  }
+  for (int i = 0; i < 3; ++i)
+    if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
+  if (args[6] != Py_None && !THPVariable_Check(args[6])) Py_RETURN_NONE;
+  const int64_t window = PyLong_AsLongLong(args[3]), n_sink = PyLong_AsLongLong(args[4]);
+  double scale = args[5] == Py_None ? 0. : PyFloat_AsDouble(args[5]);
+  if (PyErr_Occurred()) {  // numbers of other types: Python knows how to convert them, or what to raise
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+  at::Tensor q = THPVariable_Unpack(args[0]), k = THPVariable_Unpack(args[1]), v = THPVariable_Unpack(args[2]);
+  const at::Tensor cu = args[6] == Py_None ? at::Tensor() : THPVariable_Unpack(args[6]);
+  if (window < 0 || window > 0x7fffffff || n_sink < 0 || n_sink > 0x7fffffff || !ordinary(q, k, v, cu)) Py_RETURN_NONE;
+  if (args[5] == Py_None) scale = 1. / std::sqrt(static_cast<double>(q.size(-1)));
+  at::Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    q = dense(q);
+    k = dense(k);
+    v = dense(v);
+    if (k.strides() != v.strides()) {
+      k = k.contiguous();
+      v = v.contiguous();
+    }
+    if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+      out = SwaFunction::apply(q, k, v, cu.defined() ? std::optional<at::Tensor>(cu) : std::nullopt, window, n_sink, scale);
+    } else {
+      at::Tensor lse;
+      out = forward(q, k, v, cu, {window, n_sink, scale}, lse);
+    }
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// set_status(device index, address of the status word, address of its host mirror)
+PyObject* py_set_status(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3) {
+    PyErr_SetString(PyExc_TypeError, "set_status takes 3 arguments");
+    return nullptr;
+  }
+  const long dev = PyLong_AsLong(args[0]);
+  void* status = PyLong_AsVoidPtr(args[1]);
+  void* mirror = PyLong_AsVoidPtr(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (dev >= 0 && dev < kMaxDevices) {
+    g_status[dev] = static_cast<int32_t*>(status);
+    g_mirror[dev] = static_cast<const volatile int32_t*>(mirror);
+  }
+  Py_RETURN_NONE;
+}
+
+PyMethodDef g_methods[] = {
+    {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention)), METH_FASTCALL,
+     "attention(q, k, v, window, n_sink, scale, cu_seqlens) -> out or None (the call is not for this path)"},
+    {"set_status", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_set_status)), METH_FASTCALL,
+     "set_status(device_index, status_address, mirror_address)"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Single-GPU host path of ring_swa", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&g_module); }

@@ -90,6 +90,8 @@ class MergeAccParams(C.Structure):
 
 # every symbol include/rswa.h declares, with its signature
 SYMBOLS = {
+    "rswa_launch_count": (C.c_int64, []),
+    "rswa_set_status_mirror": (C.c_int, [C.c_void_p, C.c_void_p]),
     "rswa_abi_version": (C.c_int, []),
     "rswa_last_error": (C.c_char_p, []),
     "rswa_fwd": (C.c_int, [C.POINTER(FwdParams), C.c_void_p]),

@@ -30,11 +30,6 @@ class KVSpan:
         return self.k.shape[1]
 
 
-_status = {}
-
-# Number of kernels of this library launched so far (benchmarks report the count per timed region).
-launch_count = 0
-
 # When set to a list, every rswa_bwd call records three fresh timing events, appended here as raw handles
 # (start, mid, stop): start..mid brackets the dK/dV kernel, mid..stop the dQ kernel; benchmarks read them
 # with rswa_event_elapsed_ms.
@@ -44,6 +39,26 @@ fwd_events = None
 _mid_event = {}   # per (device, stream): the event a one-call ring backward records between its two kernels
 
 
+def __getattr__(name: str):
+    # Number of kernels of this library launched so far (benchmarks report the count per timed region).
+    if name == "launch_count":
+        return int(_C.lib().rswa_launch_count())
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
+def native_module():
+    """The C++ host path of single-GPU calls (csrc/rswa_torch.cpp).  Like the library itself it has no fallback."""
+    global _native
+    if _native is None:
+        _C.lib()
+        from . import _native as module
+        _native = module
+    return _native
+
+
+_native = None
+
+
 def _dev_key(device: torch.device):
     """('cuda', index) with a bare "cuda" resolved to the current device, so that every spelling of a
     device names the same status word."""
@@ -51,75 +66,59 @@ def _dev_key(device: torch.device):
     return (device.type, index)
 
 
+_status = {}    # per device: the word the kernels raise
+_mirrors = {}   # per device: its pinned host copy, written by the kernels themselves
+
+
 def status_word(device: torch.device) -> torch.Tensor:
-    """Device word the kernels raise when a bounded device-side wait runs out."""
+    """Device word the kernels raise when a bounded device-side wait runs out.
+
+    The word is sticky (kernels that start after it was raised do no work), so the host has to learn of it
+    without a synchronisation in the hot loop: a kernel that raises it or finds it raised also writes the code
+    to a word of pinned host memory, which raise_if_reported() reads when a public function is called."""
     key = _dev_key(device)
-    device = torch.device(*key)
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status[key]
+    word = _status.get(key)
+    if word is None:
+        device = torch.device(*key)
+        word = torch.zeros(1, dtype=torch.int32, device=device)
+        if not torch.cuda.is_current_stream_capturing():  # (pinned memory cannot be allocated in a capture)
+            mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
+            _C.check(_C.lib().rswa_set_status_mirror(word.data_ptr(), mirror.data_ptr()), "rswa_set_status_mirror")
+            native_module().set_status(key[1], word.data_ptr(), mirror.data_ptr())
+            _mirrors[key] = mirror
+        _status[key] = word
+    return word
+
+
+def _clear_status(device: torch.device) -> None:
+    # kernels still queued behind the failed one must have found the word raised before it is cleared, else
+    # they would report once more
+    torch.cuda.synchronize(device)
+    status_word(device).zero_()
+    mirror = _mirrors.get(_dev_key(device))
+    if mirror is not None:
+        mirror.zero_()
 
 
 def check_device_status(device: Optional[torch.device] = None) -> None:
     """Synchronises and raises if any kernel reported a device-side time-out since the last check."""
     if device is None:
         device = torch.device("cuda", torch.cuda.current_device())
-    w = status_word(device)
-    code = int(w.item())
+    code = int(status_word(device).item())
     if code != 0:
-        w.zero_()
+        _clear_status(device)
         raise RuntimeError(f"ring_swa kernel reported device-side error code {code} (a bounded wait ran out)")
 
 
-class _StatusMirror:
-    """Pinned host copy of a device's status word, refreshed asynchronously after a backward."""
-
-    def __init__(self, device: torch.device):
-        self.host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self.event = torch.cuda.Event()
-        self.pending = False
-
-
-_mirrors = {}
-
-
-def _mirror(device: torch.device) -> _StatusMirror:
-    key = _dev_key(device)
-    if key not in _mirrors:
-        _mirrors[key] = _StatusMirror(device)
-    return _mirrors[key]
-
-
-def mirror_status(device: torch.device) -> None:
-    """Enqueues a copy of the status word to pinned host memory behind the kernels launched so far.
-
-    The word is sticky on the device (kernels that start after it was raised do no work), so the
-    host has to learn of it without a synchronisation in the hot loop: the public functions call
-    this after every backward and raise_if_reported() at the start of the next call.  Skipped
-    inside a stream capture."""
-    if torch.cuda.is_current_stream_capturing():
+def raise_if_reported(device: torch.device) -> None:
+    """Raises RuntimeError if a kernel of an earlier call has reported a time-out, and clears the word so that
+    the following call runs normally."""
+    mirror = _mirrors.get(_dev_key(device))
+    if mirror is None:
         return
-    m = _mirror(device)
-    m.host.copy_(status_word(device), non_blocking=True)
-    m.event.record()
-    m.pending = True
-
-
-def raise_if_reported(device: torch.device, wait: bool = False) -> None:
-    """Raises RuntimeError if the last mirrored status word was non-zero, and clears the word so that
-    the following call runs normally.  Without `wait` a copy still in flight is left for later."""
-    m = _mirrors.get(_dev_key(device))
-    if m is None or not m.pending or torch.cuda.is_current_stream_capturing():
-        return
-    if wait:
-        m.event.synchronize()
-    elif not m.event.query():
-        return
-    m.pending = False
-    code = int(m.host[0])
-    if code != 0:
-        m.host.zero_()
-        status_word(device).zero_()
+    code = int(mirror[0])
+    if code != 0 and not torch.cuda.is_current_stream_capturing():
+        _clear_status(device)
         raise RuntimeError(f"ring_swa: a kernel of an earlier call gave up on a bounded device-side wait "
                            f"(code {code}); the results of that call are invalid. The status word has been "
                            f"cleared, later calls run normally.")
@@ -230,8 +229,6 @@ def fwd(q: torch.Tensor, spans: Sequence[KVSpan], window: int, n_sink: int, scal
     _C.check(_C.lib().rswa_fwd(C.byref(p), _stream()), "rswa_fwd")
     if fwd_events is not None:
         _C.lib().rswa_event_record(e1, _stream())
-    global launch_count
-    launch_count += 1
     return out, lse
 
 
@@ -289,9 +286,6 @@ def bwd(q: torch.Tensor, spans: Sequence[KVSpan], out: torch.Tensor, lse: torch.
             p.ev_main_mid = _C.lib().rswa_event_create()
         bwd_main_events.append((p.ev_main_start, p.ev_main_mid, p.ev_main_stop))
     _C.check(_C.lib().rswa_bwd(C.byref(p), _stream()), "rswa_bwd")
-    global launch_count
-    launch_count += ((1 if flags & _C.BWD_INIT else 0) + (1 if any(s.dk is not None for s in spans) else 0) +
-                     (1 if flags & _C.BWD_FINISH else 0))
     return workspace
 
 
@@ -348,8 +342,6 @@ def bwd_noalloc(q: torch.Tensor, spans: Sequence[KVSpan], out: torch.Tensor, lse
     p.dq_stride_b, p.dq_stride_t, p.dq_stride_h = dq.stride(0), dq.stride(1), dq.stride(2)
     p.status = status_word(q.device).data_ptr()
     _C.check(_C.lib().rswa_bwd_noalloc(C.byref(p), _stream()), "rswa_bwd_noalloc")
-    global launch_count
-    launch_count += 2 + (1 if spans else 0)
 
 
 def merge(o_a: torch.Tensor, lse_a: torch.Tensor, o_b: torch.Tensor, lse_b: torch.Tensor,
@@ -374,8 +366,6 @@ def merge(o_a: torch.Tensor, lse_a: torch.Tensor, o_b: torch.Tensor, lse_b: torc
     p.lse_a, p.lse_b, p.lse = lse_a.data_ptr(), lse_b.data_ptr(), lse_out.data_ptr()
     p.lse_stride_b, p.lse_stride_h = lse_a.stride(0), lse_a.stride(1)
     _C.check(_C.lib().rswa_merge(C.byref(p), _stream()), "rswa_merge")
-    global launch_count
-    launch_count += 1
     return out, lse_out
 
 
@@ -402,8 +392,6 @@ def merge_acc(acc_o: torch.Tensor, acc_lse: torch.Tensor, new_o: torch.Tensor, n
     p.acc_lse_stride_b, p.acc_lse_stride_h = acc_lse.stride(0), acc_lse.stride(1)
     p.new_lse_stride_b, p.new_lse_stride_h = new_lse.stride(0), new_lse.stride(1)
     _C.check(_C.lib().rswa_merge_acc(C.byref(p), _stream()), "rswa_merge_acc")
-    global launch_count
-    launch_count += 1
 
 
 def _rows(t: torch.Tensor) -> Tuple[int, int, int]:
@@ -422,8 +410,6 @@ def halo_accumulate(acc: torch.Tensor, recv: torch.Tensor) -> None:
     code = _C.DTYPE_F32 if recv.dtype == torch.float32 else _dtype_code(recv)
     _C.check(_C.lib().rswa_halo_accumulate(acc.data_ptr(), asb, recv.data_ptr(), rsb, code, B, n, _stream()),
              "rswa_halo_accumulate")
-    global launch_count
-    launch_count += 1
 
 
 def halo_accumulate_cast(dst: torch.Tensor, acc: torch.Tensor, recv: torch.Tensor) -> None:
@@ -436,8 +422,6 @@ def halo_accumulate_cast(dst: torch.Tensor, acc: torch.Tensor, recv: torch.Tenso
     code = _C.DTYPE_F32 if recv.dtype == torch.float32 else _dtype_code(recv)
     _C.check(_C.lib().rswa_halo_accumulate_cast(dst.data_ptr(), dsb, _dtype_code(dst), acc.data_ptr(), asb, recv.data_ptr(),
                                                 rsb, code, B, n, _stream()), "rswa_halo_accumulate_cast")
-    global launch_count
-    launch_count += 1
 
 
 def cast_from_f32(dst: torch.Tensor, src: torch.Tensor) -> None:
@@ -447,8 +431,6 @@ def cast_from_f32(dst: torch.Tensor, src: torch.Tensor) -> None:
     _, ssb, _ = _rows(src)
     _C.check(_C.lib().rswa_cast_from_f32(dst.data_ptr(), dsb, src.data_ptr(), ssb, _dtype_code(dst), B, n,
                                          _stream()), "rswa_cast_from_f32")
-    global launch_count
-    launch_count += 1
 
 
 def peer_put(dst_ptr: int, dst_pitch: int, src: torch.Tensor, flag_ptr: int, value: int) -> None:
@@ -459,14 +441,10 @@ def peer_put(dst_ptr: int, dst_pitch: int, src: torch.Tensor, flag_ptr: int, val
     es = src.element_size()
     _C.check(_C.lib().rswa_peer_put(dst_ptr, int(dst_pitch), src.data_ptr(), sb * es if rows > 1 else n * es, n * es, rows,
                                     flag_ptr if flag_ptr else None, int(value), _stream()), "rswa_peer_put")
-    global launch_count
-    launch_count += 1 if flag_ptr else 0
 
 
 def flag_set(flag_ptr: int, value: int) -> None:
     _C.check(_C.lib().rswa_flag_set(flag_ptr, int(value), _stream()), "rswa_flag_set")
-    global launch_count
-    launch_count += 1
 
 
 def flag_wait(flag_ptr: int, value: int, device: torch.device, timeout_s: float = 5.0) -> None:
@@ -474,8 +452,6 @@ def flag_wait(flag_ptr: int, value: int, device: torch.device, timeout_s: float 
     has not within timeout_s, the device status word is raised instead (see check_device_status)."""
     _C.check(_C.lib().rswa_flag_wait(flag_ptr, int(value), status_word(device).data_ptr(), int(timeout_s * 1e9),
                                      _stream()), "rswa_flag_wait")
-    global launch_count
-    launch_count += 1
 
 
 def selftest_mma(mode: int, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:

@@ -373,8 +373,6 @@ class RingAttn(torch.autograd.Function):
                     K.cast_from_f32(flat(dkv)[:, acc0:], flat(acc))
             for (hop, sender), n_msg in landed.items():   # the slots have been read: their senders may reuse them
                 link.release(1, hop, sender, n_msg)
-        if q4.is_cuda:
-            K.mirror_status(q4.device)
         if varlen:
             dq4, dk4, dv4 = dq4.squeeze(0), dk4.squeeze(0), dv4.squeeze(0)
         return dq4, dk4, dv4, None, None, None, None, None, None
@@ -390,6 +388,23 @@ def ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_glob
         cp_local_rank = dist.get_rank(group=cp_group)
     lens = None if chunk_lens is None else tuple(int(x) for x in chunk_lens)
     return RingCtx(cp_group, int(cp_size), int(cp_local_rank), cp_prev_global_rank, cp_next_global_rank, lens)
+
+
+def single_gpu(q, k, v, window_size: int, n_sink: int, softmax_scale: Optional[float], cu_seqlens):
+    """A call without a group, autograd included, in C++ (csrc/rswa_torch.cpp): one training step of its two
+    halves costs the host 20 us next to the autograd engine's own, 200 through RingAttn.  The public functions try
+    it before anything else; it returns None for what it leaves to the code below -- arguments that do not
+    fit together, other dtypes or devices, an error of an earlier call to report -- and when events, NVTX
+    ranges or plans are to be recorded, which only that code does."""
+    if _NVTX or _DEBUG or _phase_events is not None or K.fwd_events is not None or K.bwd_main_events is not None:
+        return None
+    return _native_attention(q, k, v, window_size, n_sink, softmax_scale, cu_seqlens)
+
+
+def _native_attention(*args):
+    global _native_attention   # resolved on the first call: importing the package must not need the library
+    _native_attention = K.native_module().attention
+    return _native_attention(*args)
 
 
 def attention(q, k, v, window_size: int, n_sink: int, softmax_scale: Optional[float],

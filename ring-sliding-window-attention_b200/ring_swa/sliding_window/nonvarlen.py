@@ -4,7 +4,7 @@ from typing import Optional
 import torch
 from torch.distributed import ProcessGroup
 
-from .._ring import attention, ring_ctx
+from .._ring import attention, ring_ctx, single_gpu
 
 
 def _check_nonvarlen(q, k, v):
@@ -34,6 +34,10 @@ def ring_sliding_window_attn(
     cp_local_rank and the previous/next global ranks default as in the reference
     (ring_swa/sliding_window/nonvarlen.py:388-395).  Returns [batch, seq_len, num_q_heads, head_dim].
     """
+    if cp_group is None:
+        out = single_gpu(q, k, v, window_size, 0, softmax_scale, None)
+        if out is not None:
+            return out
     _check_nonvarlen(q, k, v)
     ring = ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_global_rank)
     return attention(q, k, v, window_size, 0, softmax_scale, None, None, ring)

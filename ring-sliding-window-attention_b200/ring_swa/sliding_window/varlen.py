@@ -5,7 +5,7 @@ from typing import Optional, Sequence
 import torch
 from torch.distributed import ProcessGroup
 
-from .._ring import attention, ring_ctx
+from .._ring import attention, ring_ctx, single_gpu
 
 
 # Host copies of cu_seqlens tensors already seen, by tensor object: a model hands the same tensor to
@@ -37,7 +37,7 @@ def _varlen_prologue(q, k, v, cu_seqlens, cp_size, cp_chunk_lens=None):
     if q.is_cuda and synced:
         # the copy above has synchronised with the device anyway: a good moment to look at the status word
         from .. import _kernels
-        _kernels.raise_if_reported(q.device, wait=True)
+        _kernels.raise_if_reported(q.device)
     # ring_swa/sliding_window/varlen.py:401-403; evaluated before cp_group is looked at, so a
     # missing cp_size raises TypeError there as well
     if cp_chunk_lens is None:
@@ -79,6 +79,10 @@ def ring_sliding_window_attn_varlen(
     [sum(lens[:i]), sum(lens[:i+1])) and seq_len is its own entry.
     """
     cu_seqlens, cu_host = _varlen_prologue(q, k, v, cu_seqlens, cp_size, cp_chunk_lens)
+    if cp_group is None:
+        out = single_gpu(q, k, v, window_size, 0, softmax_scale, cu_seqlens)
+        if out is not None:
+            return out
     ring = ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_global_rank, cp_chunk_lens)
     return attention(q, k, v, window_size, 0, softmax_scale, cu_seqlens, cu_host, ring)
 

@@ -4,7 +4,7 @@ from typing import Optional
 import torch
 from torch.distributed import ProcessGroup
 
-from .._ring import attention, ring_ctx
+from .._ring import attention, ring_ctx, single_gpu
 from ..sliding_window.nonvarlen import _check_nonvarlen
 
 
@@ -30,6 +30,10 @@ def ring_streaming_llm_attn(
     own first token (the reference takes batch row 0's for every row, which is the same under its
     stated assumption that all sinks are identical).
     """
+    if cp_group is None:
+        out = single_gpu(q, k, v, window_size, num_sink_tokens, softmax_scale, None)
+        if out is not None:
+            return out
     _check_nonvarlen(q, k, v)
     ring = ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_global_rank)
     return attention(q, k, v, window_size, num_sink_tokens, softmax_scale, None, None, ring)

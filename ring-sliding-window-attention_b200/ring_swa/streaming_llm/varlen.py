@@ -4,7 +4,7 @@ from typing import Optional, Sequence
 import torch
 from torch.distributed import ProcessGroup
 
-from .._ring import attention, ring_ctx
+from .._ring import attention, ring_ctx, single_gpu
 from ..sliding_window.varlen import _varlen_prologue
 
 
@@ -34,6 +34,10 @@ def ring_streaming_llm_attn_varlen(
     `cp_chunk_lens`: chunks of different lengths per rank, as in ring_sliding_window_attn_varlen.
     """
     cu_seqlens, cu_host = _varlen_prologue(q, k, v, cu_seqlens, cp_size, cp_chunk_lens)
+    if cp_group is None:
+        out = single_gpu(q, k, v, window_size, num_sink_tokens, softmax_scale, cu_seqlens)
+        if out is not None:
+            return out
     ring = ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_global_rank, cp_chunk_lens)
     return attention(q, k, v, window_size, num_sink_tokens, softmax_scale, cu_seqlens, cu_host, ring)
 
