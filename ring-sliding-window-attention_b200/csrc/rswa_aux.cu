@@ -41,6 +41,7 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
                              const float* __restrict__ lse, long long l_sb, long long l_sh,
                              float* __restrict__ delta, float* __restrict__ lse2, int batch, int q_len, int hq,
                              int q_len_pad, int* __restrict__ counters) {
+  griddep_launch();  // (to the dK/dV kernel, which waits for this one)
   // the work counters of the two kernels behind this one (a memset of 8 bytes would be a launch of its own)
   if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // warp task

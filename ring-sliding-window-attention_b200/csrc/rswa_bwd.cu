@@ -101,8 +101,6 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
   float* sDelta = sLse + kQStages * kTile;                       // [2][128], travels with dO
   BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem + kBwdSmemTiles + (kQStages + 2) * kRowBytes);
 
-  if (status_raised(p.status, p.mirror)) return;
-
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int group = p.hq / p.hkv;
@@ -127,7 +125,6 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
     mbar_init(&ctl->dp_ready, 1);
     mbar_init(&ctl->done, 1);
     mbar_init(&ctl->acc_free, kComputeThreads / 32);
-    ctl->err = (smem_u32(smem) & 1023u) ? 199 : 0;
     mbar_fence_init();
     prefetch_tmap(&p.q_map);
     prefetch_tmap(&p.do_map);
@@ -136,6 +133,10 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
     tmem_alloc(&ctl->tmem_base, kBwdTmemCols);
     tmem_relinquish();
   }
+  // (behind the wait, not in front of it: the dQ kernel relies on the delta kernel having finished)
+  griddep_wait();
+  griddep_launch();
+  if (threadIdx.x == 0) ctl->err = (smem_u32(smem) & 1023u) ? 199 : status_code(p.status, p.mirror);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ B
 
 }  // namespace
 
-int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaStream_t stream) {
+int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool early, cudaStream_t stream) {
   // far items (see BwdKernelParams) come first: they are the longest where the segments' sequences are long
   const long long n_cta = (static_cast<long long>(total_key_tiles) + static_cast<long long>(kp.far_segs) * kp.n_spans) * kp.hkv * kp.batch;
   if (n_cta <= 0) return RSWA_OK;
@@ -691,19 +692,24 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, cudaSt
   }
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_grid = n_cta < sm_count() ? n_cta : sm_count();
-  kern<<<static_cast<unsigned>(n_grid), kBwdThreads, kBwdSmemBytes, stream>>>(kp, static_cast<int>(n_cta));
-  count_launches(kp.far_segs > 0 ? 2 : 1);
-  e = cudaGetLastError();
+  e = launch_kernel(kern, dim3(static_cast<unsigned>(n_grid)), kBwdThreads, kBwdSmemBytes, stream, early, kp, static_cast<int>(n_cta));
+  count_launches(1);
   if (e != cudaSuccess) {
     set_error("rswa_bwd: launch: %s", cudaGetErrorString(e));
     return RSWA_E_CUDA;
   }
+  return RSWA_OK;
+}
+
+// Adds the sink rows' partial sums up, behind the dK/dV kernel (not necessarily right behind it).
+int launch_sink_sum(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
   if (kp.far_segs > 0) {
     const int n_seq = kp.cu == nullptr ? 1 : kp.n_seqs + 1;
     const dim3 grid(static_cast<unsigned>(n_seq * kp.n_sink), static_cast<unsigned>(kp.hkv), static_cast<unsigned>(kp.batch));
     if (dtype == RSWA_DTYPE_BF16) sink_sum_kernel<true><<<grid, 256, 0, stream>>>(kp);
     else sink_sum_kernel<false><<<grid, 256, 0, stream>>>(kp);
-    e = cudaGetLastError();
+    count_launches(1);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
       set_error("rswa_bwd: sink sums: launch: %s", cudaGetErrorString(e));
       return RSWA_E_CUDA;

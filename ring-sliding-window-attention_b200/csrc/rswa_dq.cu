@@ -100,8 +100,6 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
   uint8_t* sV = smem + 5 * kTileBytes;  // two stages
   DqCtl* ctl = reinterpret_cast<DqCtl*>(smem + kDqSmemTiles);
 
-  if (status_raised(p.status, p.mirror)) return;
-
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -127,7 +125,10 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
     mbar_init(&ctl->ds_ready, kDqCompute / 32);  // one arrival per compute warp
     mbar_init(&ctl->done, 1);
     mbar_init(&ctl->dq_drained, kDqCompute / 32);  // one arrival per compute warp
-    ctl->err = (smem_u32(smem) & 1023u) ? 199 : 0;
+    // No griddep_wait() here: when this kernel starts early, the kernel it overlaps is the dK/dV kernel of the same
+    // call, which it needs nothing from and which lets it start only after the delta kernel, and with it everything
+    // that came before the call, has finished.  The wait is at the end instead.
+    ctl->err = (smem_u32(smem) & 1023u) ? 199 : status_code(p.status, p.mirror);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -538,12 +539,14 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
     tc_fence_after();
     tmem_dealloc(tmem, kDqTmemCols);
   }
+  // (this kernel must not be finished before the dK/dV kernel is: what follows on the stream waits for this one)
+  griddep_wait();
   if (threadIdx.x == 0 && ctl->err != 0) raise_status(p.status, p.mirror, ctl->err);
 }
 
 }  // namespace
 
-int launch_dq(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
+int launch_dq(const BwdKernelParams& kp, int dtype, bool early, cudaStream_t stream) {
   const int n_q_tiles = (kp.q_len + kTile - 1) / kTile;
   const long long n_items = static_cast<long long>(n_q_tiles) * kp.hq * kp.batch;
   if (n_items <= 0) return RSWA_OK;
@@ -571,9 +574,8 @@ int launch_dq(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
   }
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_cta = n_items < sm_count() ? n_items : sm_count();
-  kern<<<static_cast<unsigned>(n_cta), kDqThreads, kDqSmemBytes, stream>>>(kp, n_q_tiles, static_cast<int>(n_items));
+  e = launch_kernel(kern, dim3(static_cast<unsigned>(n_cta)), kDqThreads, kDqSmemBytes, stream, early, kp, n_q_tiles, static_cast<int>(n_items));
   count_launches(1);
-  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rswa_bwd(dq): launch: %s", cudaGetErrorString(e));
     return RSWA_E_CUDA;

@@ -124,8 +124,6 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
   FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem + kFwdSmemTiles);
 
   RSWA_TRC(fwd, threadIdx.x == 0, 1920);
-  if (status_raised(p.status, p.mirror)) return;
-
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -145,13 +143,14 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
       mbar_init(&ctl->geom_full[i], 1);
       mbar_init(&ctl->geom_free[i], kSoftmaxWarps);
     }
-    ctl->err = (smem_u32(smem) & 1023u) ? 199 : 0;
     mbar_fence_init();
   }
   if (warp == 1) {
     tmem_alloc(&ctl->tmem_base, kFwdTmemCols);
     tmem_relinquish();
   }
+  griddep_wait();
+  if (threadIdx.x == 0) ctl->err = (smem_u32(smem) & 1023u) ? 199 : status_code(p.status, p.mirror);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -675,9 +674,8 @@ int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream) {
   }
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_cta = n_items < sm_count() ? n_items : sm_count();
-  kern<<<static_cast<unsigned>(n_cta), kFwdThreads, kFwdSmemBytes, stream>>>(kp, n_blocks, static_cast<int>(n_items));
+  e = launch_kernel(kern, dim3(static_cast<unsigned>(n_cta)), kFwdThreads, kFwdSmemBytes, stream, true, kp, n_blocks, static_cast<int>(n_items));
   count_launches(1);
-  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rswa_fwd: launch: %s", cudaGetErrorString(e));
     return RSWA_E_CUDA;

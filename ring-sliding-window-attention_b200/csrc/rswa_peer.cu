@@ -31,7 +31,7 @@ __global__ void flag_set_kernel(int* flag, int value) {
 }
 
 __global__ void flag_wait_kernel(const int* flag, int value, int* status, int* mirror, unsigned long long timeout_ns) {
-  if (status_raised(status, mirror)) return;
+  if (status_code(status, mirror) != 0) return;
   unsigned long long t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   for (;;) {

@@ -367,3 +367,48 @@ def test_peer_put_and_bounded_flag_wait():
     K.flag_set(flags[1:].data_ptr(), 1)
     K.flag_wait(flags[1:].data_ptr(), 1, dev, timeout_s=2.0)
     K.check_device_status()
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,W,n_sink", [
+    (1, 100, 2, 1, 40, 0),      # one work item: the dQ kernel starts at once beside it
+    (1, 4096, 16, 1, 1000, 0),  # 32 long dK/dV items: most SMs are left to the dQ kernel, which finishes its work first
+    (2, 3001, 16, 2, 500, 1),   # sink sums behind both kernels
+    (2, 2048, 16, 16, 128, 0),  # more items than SMs
+])
+def test_overlapped_backward_kernels_finish_together(B, S, Hq, Hkv, W, n_sink):
+    """The dQ kernel starts while the dK/dV kernel still runs; a call with an event between the two keeps them
+    apart.  Nothing is reduced across CTAs, so the results are the same bits, also for what follows on the stream
+    without a synchronisation, when the buffers are used again, and in a captured graph."""
+    K = _K()
+    dev = torch.device("cuda")
+    q, k, v, do = (randn_bf16(B, S, h, D, seed=s).to(dev) for h, s in ((Hq, 1), (Hkv, 2), (Hkv, 3), (Hq, 4)))
+    out, lse = K.fwd(q, [K.KVSpan(k, v, 0)], W, n_sink, D ** -0.5)
+    ws = K.bwd_workspace(q, Hkv, W, n_sink)
+
+    def bwd(dq, dk, dv, **kw):
+        K.bwd(q, [K.KVSpan(k, v, 0, dk, dv)], out, lse, do, dq, W, n_sink, D ** -0.5, workspace=ws, **kw)
+
+    ref = [torch.empty_like(x) for x in (q, k, v)]
+    bwd(*ref, mid_event=K.mid_event_for(dev))
+    grads = [torch.empty_like(x) for x in (q, k, v)]
+    copies = []
+    for _ in range(6):
+        for x in grads:
+            x.fill_(float("nan"))
+        bwd(*grads)
+        copies.append([x.clone() for x in grads])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        for x in grads:
+            x.fill_(float("nan"))
+        bwd(*grads)
+        captured = [x + 0 for x in grads]
+    for _ in range(3):
+        graph.replay()
+        copies.append([x.clone() for x in captured])
+    K.check_device_status()
+    for got in copies:
+        for name, a, b in zip(("dq", "dk", "dv"), got, ref):
+            assert torch.equal(a, b), name
