@@ -104,6 +104,8 @@ typedef struct rswa_fwd_params {
 } rswa_fwd_params_t;
 
 int rswa_fwd(const rswa_fwd_params_t* p, void* stream);
+/* The same for heads of 64 elements (head_dim must be 64; `carry` is not available). */
+int rswa_fwd_d64(const rswa_fwd_params_t* p, void* stream);
 
 /* Backward: dq [batch,q_len,Hq,D] and per-span dk/dv from (dO, q, spans, out, lse), using the
  * final (merged) out and lse.  Two kernels: a key-stationary one writes dk/dv of every span that
@@ -151,6 +153,9 @@ int64_t rswa_bwd_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_q_heads
 int64_t rswa_bwd_sink_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_kv_heads, int32_t window,
                                       int32_t n_sink, int32_t n_seqs);
 int rswa_bwd(const rswa_bwd_params_t* p, void* stream);
+/* The same for heads of 64 elements (head_dim must be 64).  The workspace is the one of 128-wide heads:
+ * rswa_bwd_workspace_bytes(batch, q_len, n_q_heads, 128). */
+int rswa_bwd_d64(const rswa_bwd_params_t* p, void* stream);
 
 /* The whole backward for callers that cannot allocate device memory: same inputs, outputs and
  * result as rswa_bwd with flags INIT|FINISH, but `workspace`, `workspace_bytes` and `flags` are

@@ -72,10 +72,10 @@ static EncodeTiledFn get_encode() {
 namespace {
 struct MapKey {
   const void* base;
-  int dtype, batch, tokens, heads;
+  int dtype, batch, tokens, heads, head_dim;
   long long sb, st, sh;
   bool operator==(const MapKey& o) const {
-    return base == o.base && dtype == o.dtype && batch == o.batch && tokens == o.tokens && heads == o.heads &&
+    return base == o.base && dtype == o.dtype && batch == o.batch && tokens == o.tokens && heads == o.heads && head_dim == o.head_dim &&
            sb == o.sb && st == o.st && sh == o.sh;
   }
 };
@@ -88,7 +88,7 @@ struct MapCache {
 thread_local MapCache t_map_cache;
 }  // namespace
 
-int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int tokens, int heads,
+int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int tokens, int heads, int head_dim,
                   long long sb, long long st, long long sh) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return RSWA_E_CUDA;
@@ -114,7 +114,7 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int 
     return RSWA_E_ARG;
   }
   if (batch == 1 && sb == 0) sb = static_cast<long long>(tokens) * st;
-  const MapKey key{base, dtype, batch, tokens, heads, sb, st, sh};
+  const MapKey key{base, dtype, batch, tokens, heads, head_dim, sb, st, sh};
   MapCache& cache = t_map_cache;
   for (int i = 0; i < cache.used; ++i) {
     if (cache.key[i] == key) {
@@ -122,7 +122,7 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int 
       return RSWA_OK;
     }
   }
-  cuuint64_t dims[4] = {static_cast<cuuint64_t>(kHeadDim), static_cast<cuuint64_t>(heads),
+  cuuint64_t dims[4] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(heads),
                         static_cast<cuuint64_t>(tokens), static_cast<cuuint64_t>(batch)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(sh) * 2, static_cast<cuuint64_t>(st) * 2,
                            static_cast<cuuint64_t>(sb) * 2};
@@ -143,13 +143,13 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int 
   return RSWA_OK;
 }
 
-int check_geom(const rswa_geom_t& g, bool need_grads) {
+int check_geom(const rswa_geom_t& g, bool need_grads, int head_dim) {
   if (g.dtype != RSWA_DTYPE_BF16 && g.dtype != RSWA_DTYPE_FP16) {
     set_error("dtype must be bf16 (0) or fp16 (1), got %d", g.dtype);
     return RSWA_E_UNSUPPORTED;
   }
-  if (g.head_dim != kHeadDim) {
-    set_error("head_dim must be %d, got %d", kHeadDim, g.head_dim);
+  if (g.head_dim != head_dim) {
+    set_error("head_dim must be %d, got %d", head_dim, g.head_dim);
     return RSWA_E_UNSUPPORTED;
   }
   if (g.batch <= 0 || g.q_len <= 0 || g.n_q_heads <= 0 || g.n_kv_heads <= 0) {
@@ -204,10 +204,10 @@ int check_geom(const rswa_geom_t& g, bool need_grads) {
 static int fill_span_maps(const rswa_geom_t& g, CUtensorMap* kmaps, CUtensorMap* vmaps, int* pos, int* len) {
   for (int i = 0; i < g.n_spans; ++i) {
     const rswa_span_t& s = g.spans[i];
-    int rc = make_tile_map(&kmaps[i], s.k, g.dtype, g.batch, s.len, g.n_kv_heads, s.kv_stride_b, s.kv_stride_t,
+    int rc = make_tile_map(&kmaps[i], s.k, g.dtype, g.batch, s.len, g.n_kv_heads, g.head_dim, s.kv_stride_b, s.kv_stride_t,
                            s.kv_stride_h);
     if (rc) return rc;
-    rc = make_tile_map(&vmaps[i], s.v, g.dtype, g.batch, s.len, g.n_kv_heads, s.kv_stride_b, s.kv_stride_t,
+    rc = make_tile_map(&vmaps[i], s.v, g.dtype, g.batch, s.len, g.n_kv_heads, g.head_dim, s.kv_stride_b, s.kv_stride_t,
                        s.kv_stride_h);
     if (rc) return rc;
     pos[i] = s.pos_start;
@@ -277,13 +277,13 @@ extern "C" int rswa_set_status_mirror(const int32_t* status, int32_t* mirror) {
   return RSWA_OK;
 }
 
-extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
+static int fwd_call(const rswa_fwd_params_t* p, int head_dim, void* stream) {
   if (p == nullptr) {
     set_error("rswa_fwd: null params");
     return RSWA_E_ARG;
   }
   const rswa_geom_t& g = p->g;
-  int rc = check_geom(g, false);
+  int rc = check_geom(g, false, head_dim);
   if (rc) return rc;
   if (p->q == nullptr || p->out == nullptr || p->lse == nullptr || p->status == nullptr) {
     set_error("rswa_fwd: q, out, lse and status are required");
@@ -293,6 +293,10 @@ extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
     set_error("rswa_fwd: out must be 16-byte aligned with strides that are multiples of 8 elements");
     return RSWA_E_ARG;
   }
+  if (p->carry != 0 && head_dim != kHeadDim) {
+    set_error("rswa_fwd: a partial result can only be continued with head_dim %d", kHeadDim);
+    return RSWA_E_UNSUPPORTED;
+  }
   const int n_tiles_all = (g.q_len + kTile - 1) / kTile;
   int qb = p->q_tile_begin, qe = p->q_tile_end <= 0 ? n_tiles_all : p->q_tile_end;
   if (qb < 0 || qe > n_tiles_all || qb > qe) {
@@ -301,7 +305,7 @@ extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
   }
   FwdKernelParams kp;
   memset(&kp, 0, sizeof(kp));
-  rc = make_tile_map(&kp.q_map, p->q, g.dtype, g.batch, g.q_len, g.n_q_heads, p->q_stride_b, p->q_stride_t,
+  rc = make_tile_map(&kp.q_map, p->q, g.dtype, g.batch, g.q_len, g.n_q_heads, head_dim, p->q_stride_b, p->q_stride_t,
                      p->q_stride_h);
   if (rc) return rc;
   rc = fill_span_maps(g, kp.k_map, kp.v_map, kp.span_pos, kp.span_len);
@@ -311,6 +315,7 @@ extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
   kp.q_len = g.q_len;
   kp.hq = g.n_q_heads;
   kp.hkv = g.n_kv_heads;
+  kp.head_dim = head_dim;
   kp.q_pos_start = g.q_pos_start;
   kp.window = g.window;
   kp.n_sink = g.n_sink;
@@ -332,6 +337,9 @@ extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) {
   return launch_fwd(kp, g.dtype, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int rswa_fwd(const rswa_fwd_params_t* p, void* stream) { return fwd_call(p, kHeadDim, stream); }
+extern "C" int rswa_fwd_d64(const rswa_fwd_params_t* p, void* stream) { return fwd_call(p, kNarrowHeadDim, stream); }
+
 extern "C" int64_t rswa_bwd_workspace_bytes(int32_t batch, int32_t q_len, int32_t n_q_heads, int32_t head_dim) {
   if (batch <= 0 || q_len <= 0 || n_q_heads <= 0 || head_dim != kHeadDim) return -1;
   const int64_t q_len_pad = (static_cast<int64_t>(q_len) + kTile - 1) / kTile * kTile;
@@ -346,14 +354,14 @@ extern "C" int64_t rswa_bwd_sink_workspace_bytes(int32_t batch, int32_t q_len, i
   return far_plan(batch, q_len, n_kv_heads, window, n_sink, n_seqs).bytes;
 }
 
-extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
+static int bwd_call(const rswa_bwd_params_t* p, int head_dim, void* stream_) {
   if (p == nullptr) {
     set_error("rswa_bwd: null params");
     return RSWA_E_ARG;
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const rswa_geom_t& g = p->g;
-  int rc = check_geom(g, false);
+  int rc = check_geom(g, false, head_dim);
   if (rc) return rc;
   if (!p->q || !p->out || !p->dout || !p->lse || !p->workspace || !p->status) {
     set_error("rswa_bwd: q, out, dout, lse, workspace and status are required");
@@ -364,7 +372,7 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
     set_error("rswa_bwd: dq is required with RSWA_BWD_FINISH");
     return RSWA_E_ARG;
   }
-  const int64_t need = rswa_bwd_workspace_bytes(g.batch, g.q_len, g.n_q_heads, g.head_dim);
+  const int64_t need = rswa_bwd_workspace_bytes(g.batch, g.q_len, g.n_q_heads, kHeadDim);
   if (p->workspace_bytes < need || (reinterpret_cast<uintptr_t>(p->workspace) & 255) != 0) {
     set_error("rswa_bwd: workspace needs %lld bytes, 256-byte aligned (got %lld)", (long long)need,
               (long long)p->workspace_bytes);
@@ -390,10 +398,10 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   // kq: every span (the dQ kernel sums over all keys); kk: only the spans whose dK/dV are wanted
   BwdKernelParams kq, kk;
   memset(&kq, 0, sizeof(kq));
-  rc = make_tile_map(&kq.q_map, p->q, g.dtype, g.batch, g.q_len, g.n_q_heads, p->q_stride_b, p->q_stride_t,
+  rc = make_tile_map(&kq.q_map, p->q, g.dtype, g.batch, g.q_len, g.n_q_heads, head_dim, p->q_stride_b, p->q_stride_t,
                      p->q_stride_h);
   if (rc) return rc;
-  rc = make_tile_map(&kq.do_map, p->dout, g.dtype, g.batch, g.q_len, g.n_q_heads, p->do_stride_b,
+  rc = make_tile_map(&kq.do_map, p->dout, g.dtype, g.batch, g.q_len, g.n_q_heads, head_dim, p->do_stride_b,
                      p->do_stride_t, p->do_stride_h);
   if (rc) return rc;
   rc = fill_span_maps(g, kq.k_map, kq.v_map, kq.span_pos, kq.span_len);
@@ -403,6 +411,7 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   kq.q_len = g.q_len;
   kq.hq = g.n_q_heads;
   kq.hkv = g.n_kv_heads;
+  kq.head_dim = head_dim;
   kq.q_pos_start = g.q_pos_start;
   kq.window = g.window;
   kq.n_sink = g.n_sink;
@@ -486,6 +495,9 @@ extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream_) {
   if (p->ev_main_stop) cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_stop), stream);
   return RSWA_OK;
 }
+
+extern "C" int rswa_bwd(const rswa_bwd_params_t* p, void* stream) { return bwd_call(p, kHeadDim, stream); }
+extern "C" int rswa_bwd_d64(const rswa_bwd_params_t* p, void* stream) { return bwd_call(p, kNarrowHeadDim, stream); }
 
 extern "C" void* rswa_event_create(void) {
   cudaEvent_t ev = nullptr;

@@ -30,12 +30,12 @@ __device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
   }
 }
 
-// A warp takes 32 consecutive tokens of one (batch row, head): half a warp per 128-element row (16 bytes
-// per lane and tensor), eight rows in flight per lane pair, and the 32 results leave as ONE 128-byte
+// A warp takes 32 consecutive tokens of one (batch row, head): 16 lanes per 128-element row (16 bytes per lane and
+// tensor; 8 lanes per 64-element row), eight loads of each tensor in flight per lane, and the 32 results leave as ONE 128-byte
 // segment of each output row (one token per lane) instead of 32 scattered words.  Writes
 // -delta = -rowsum(dO * O) and -lse2 = -lse * log2(e) into rows padded to whole 128-query tiles; the
 // padding gets -delta = 0 and -lse2 = -inf so that P = exp2(s - lse2) vanishes there.
-template <bool kBf16>
+template <int kD, bool kBf16>
 __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, long long o_st, long long o_sh,
                              const uint16_t* __restrict__ dout, long long d_sb, long long d_st, long long d_sh,
                              const float* __restrict__ lse, long long l_sb, long long l_sh,
@@ -46,7 +46,8 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
   if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // warp task
   const int lane = threadIdx.x & 31;
-  const int sub = lane & 15, hi = lane >> 4;
+  constexpr int kLanes = kD / 8, kRows = 32 / kLanes;  // lanes per row, rows per load
+  const int sub = lane % kLanes, hi = lane / kLanes;
   const int t_blocks = q_len_pad >> 5;  // q_len_pad is a multiple of 128
   const long long n_tasks = static_cast<long long>(batch) * hq * t_blocks;
   if (wid >= n_tasks) return;
@@ -59,11 +60,11 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
   const uint16_t* pd = dout + b * d_sb + h * d_sh + sub * 8;
   float mine = 0.f;  // the sum of the token this lane will write (t0 + lane)
 #pragma unroll
-  for (int blk = 0; blk < 2; ++blk) {  // 16 tokens per block: 8 loads of each tensor in flight per lane
+  for (int blk = 0; blk < 4 / kRows; ++blk) {  // 8 loads of each tensor in flight per lane
     uint4 a[8], d[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int t = t0 + blk * 16 + 2 * i + hi;
+      const int t = t0 + (blk * 8 + i) * kRows + hi;
       if (t < q_len) {
         a[i] = *reinterpret_cast<const uint4*>(po + t * o_st);
         d[i] = *reinterpret_cast<const uint4*>(pd + t * d_st);
@@ -82,11 +83,13 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
         s += x.x * y.x + x.y * y.y;
       }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      // lanes 0-15 hold the sum of token t0 + 16 blk + 2 i, lanes 16-31 that of the next one
-      const float lo_sum = __shfl_sync(0xffffffffu, s, 0), hi_sum = __shfl_sync(0xffffffffu, s, 16);
-      if (lane == blk * 16 + 2 * i) mine = lo_sum;
-      if (lane == blk * 16 + 2 * i + 1) mine = hi_sum;
+      for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      // each group of lanes holds the sum of one of kRows consecutive tokens
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const float sum = __shfl_sync(0xffffffffu, s, r * kLanes);
+        if (lane == (blk * 8 + i) * kRows + r) mine = sum;
+      }
     }
   }
   const int t = t0 + lane;
@@ -333,7 +336,9 @@ int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_le
   const long long tasks = static_cast<long long>(g.batch) * g.n_q_heads * (q_len_pad / 32);  // one warp each
   const int threads = 256;
   const long long blocks = (tasks * 32 + threads - 1) / threads;
-  auto kern = g.dtype == RSWA_DTYPE_BF16 ? delta_kernel<true> : delta_kernel<false>;
+  const bool narrow = g.head_dim == kNarrowHeadDim;
+  auto kern = g.dtype == RSWA_DTYPE_BF16 ? (narrow ? delta_kernel<64, true> : delta_kernel<128, true>)
+                                         : (narrow ? delta_kernel<64, false> : delta_kernel<128, false>);
   kern<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
       static_cast<const uint16_t*>(p.out), p.o_stride_b, p.o_stride_t, p.o_stride_h,
       static_cast<const uint16_t*>(p.dout), p.do_stride_b, p.do_stride_t, p.do_stride_h, p.lse, p.lse_stride_b,

@@ -77,7 +77,6 @@ struct BwdCtl {
 constexpr int kBwdSmemTiles = 7 * kTileBytes;
 constexpr int kRowBytes = kTile * 4;
 constexpr int kBwdSmemBytes = kBwdSmemTiles + (kQStages + 2) * kRowBytes + 512;
-constexpr uint32_t kStageTxBytes = kTileBytes + kRowBytes;
 constexpr int kGeomUsers = 1 + kComputeThreads / 32;  // the MMA thread and one lane per compute warp
 static_assert(sizeof(BwdCtl) <= 512, "control block too large");
 static_assert(kBwdSmemBytes <= 232448, "shared memory budget");
@@ -85,9 +84,12 @@ static_assert(kBwdSmemBytes <= 232448, "shared memory budget");
 // kPlain: one KV span, no packed sequences, no sink tokens, 16-bit gradients (the plain sliding window
 // of one GPU): what such a call cannot need is compiled out of its variant (the SM's instruction
 // cache holds 32 KB).
-template <bool kBf16, bool kPlain>
+// kD: width of a head, 128 or 64.
+template <int kD, bool kBf16, bool kPlain>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
+  constexpr uint32_t kLoadBytes = kD / 64 * kBoxBytes;  // what a tile holds (its slots in shared memory are kTileBytes apart)
+  constexpr uint32_t kStageTxBytes = kLoadBytes + kRowBytes;
   const int* const cu_seq = kPlain ? nullptr : p.cu;
   const int n_seqs = kPlain ? 0 : p.n_seqs;
   const int n_spans = kPlain ? 1 : p.n_spans;
@@ -222,11 +224,11 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         // K and V have one buffer each: the previous item's last S^T and dP^T products must have read them
         if (nk > 0 && !mbar_wait<200>(&ctl->kv_free, (nk - 1) & 1, err, kErrWaitProducer)) break;
         ++nk;
-        mbar_expect_tx(&ctl->kv_full, 2 * kTileBytes);
+        mbar_expect_tx(&ctl->kv_full, 2 * kLoadBytes);
         tma_load_4d(sK, &p.k_map[sp], &ctl->kv_full, 0, hk, key0, b);
-        tma_load_4d(sK + kBoxBytes, &p.k_map[sp], &ctl->kv_full, 64, hk, key0, b);
+        if (kD > 64) tma_load_4d(sK + kBoxBytes, &p.k_map[sp], &ctl->kv_full, 64, hk, key0, b);
         tma_load_4d(sV, &p.v_map[sp], &ctl->kv_full, 0, hk, key0, b);
-        tma_load_4d(sV + kBoxBytes, &p.v_map[sp], &ctl->kv_full, 64, hk, key0, b);
+        if (kD > 64) tma_load_4d(sV + kBoxBytes, &p.v_map[sp], &ctl->kv_full, 64, hk, key0, b);
         bool ok = true;
         for (int ih = 0; ih < group && ok; ++ih) {
           const int h = hk * group + ih;
@@ -239,13 +241,13 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
             if (!ok) break;
             mbar_expect_tx(&ctl->q_full[sq], kStageTxBytes);
             tma_load_4d(sQ + sq * kTileBytes, &p.q_map, &ctl->q_full[sq], 0, h, row0, b);
-            tma_load_4d(sQ + sq * kTileBytes + kBoxBytes, &p.q_map, &ctl->q_full[sq], 64, h, row0, b);
+            if (kD > 64) tma_load_4d(sQ + sq * kTileBytes + kBoxBytes, &p.q_map, &ctl->q_full[sq], 64, h, row0, b);
             bulk_load_1d(sLse + sq * kTile, p.lse2 + roff, kRowBytes, &ctl->q_full[sq]);
             if (gi >= 2) ok = mbar_wait<200>(&ctl->do_free[sd], ((gi >> 1) - 1) & 1, err, kErrWaitProducer);
             if (!ok) break;
             mbar_expect_tx(&ctl->do_full[sd], kStageTxBytes);
             tma_load_4d(sDO + sd * kTileBytes, &p.do_map, &ctl->do_full[sd], 0, h, row0, b);
-            tma_load_4d(sDO + sd * kTileBytes + kBoxBytes, &p.do_map, &ctl->do_full[sd], 64, h, row0, b);
+            if (kD > 64) tma_load_4d(sDO + sd * kTileBytes + kBoxBytes, &p.do_map, &ctl->do_full[sd], 64, h, row0, b);
             bulk_load_1d(sDelta + sd * kTile, p.delta + roff, kRowBytes, &ctl->do_full[sd]);
           }
         }
@@ -263,7 +265,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
       // dV / dK of this one directly: its K and V were loaded while this item's last tiles ran.
       constexpr int bf = kBf16 ? 1 : 0;
       constexpr uint32_t id_kk = idesc_f16(128, 128, bf, 0, 0);  // both operands K-major
-      constexpr uint32_t id_tn = idesc_f16(128, 128, bf, 0, 1);  // A from TMEM, B MN-major
+      constexpr uint32_t id_tn = idesc_f16(128, kD, bf, 0, 1);  // A from TMEM, B MN-major
       const uint64_t dK = smem_desc_sw128(smem_u32(sK), 16, 1024);
       const uint64_t dV = smem_desc_sw128(smem_u32(sV), 16, 1024);
       const uint64_t dQk = smem_desc_sw128(smem_u32(sQ), 16, 1024);
@@ -337,7 +339,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
             tc_fence_after();
             const uint64_t dDOs = dDOk + sd * kTile16;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < kD / 16; ++k) {
               const uint32_t off = ((k >> 2) * kBoxBytes + (k & 3) * 32) >> 4;
               mma_ss(tB, dV + off, dDOs + off, id_kk, k > 0 ? 1u : 0u);
             }
@@ -353,7 +355,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
             tc_fence_after();
             const uint64_t dQs = dQk + sq * kTile16;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < kD / 16; ++k) {
               const uint32_t off = ((k >> 2) * kBoxBytes + (k & 3) * 32) >> 4;
               mma_ss(tS, dK + off, dQs + off, id_kk, k > 0 ? 1u : 0u);
             }
@@ -378,10 +380,10 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
     // of the NEXT item: its last products are still running when its last dS^T has been handed over
     // (waiting for them right there left every compute warp idle), and the next item's first dV / dK
     // products are a whole tile's work away.  32 columns at a time through ONE copy of the code (a
-    // thread owns 64 consecutive columns of one key row: 32-byte stores, whole sectors).
+    // thread owns kD / 2 consecutive columns of one key row: 32-byte stores, whole sectors).
     bool pend = false;
     int pend_nk = 0, pend_sp = 0;
-    long long pend_off = -1;  // element offset of this thread's 64 columns (-1: the key row does not exist)
+    long long pend_off = -1;  // element offset of this thread's columns (-1: the key row does not exist)
     float* pend_ws = nullptr;  // partial sums of a sink row (non-null: this row does not go to dk / dv)
     auto drain = [&]() -> bool {
       bool k = mbar_wait(&ctl->done, pend_nk & 1, err, kErrWaitEpilogue);
@@ -390,10 +392,10 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
       tc_fence_after();
       const bool f32 = !kPlain && p.grad_fp32[pend_sp] != 0;
 #pragma unroll 1
-      for (int wc = 0; wc < 4; ++wc) {
-        const int which = wc >> 1, c = wc & 1;
+      for (int wc = 0; wc < kD / 32; ++wc) {
+        const int which = kD > 64 ? wc >> 1 : wc, c = kD > 64 ? wc & 1 : 0;
         uint32_t r[32];
-        tmem_ld32((which == 0 ? tDK : tDV) + lane_off + half * 64 + c * 32, r);
+        tmem_ld32((which == 0 ? tDK : tDV) + lane_off + half * (kD / 2) + c * 32, r);
         tmem_ld_wait();
         const float mul = which == 0 ? p.scale : 1.f;
         void* base = which == 0 ? p.dk[pend_sp] : p.dv[pend_sp];
@@ -450,7 +452,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         p_hi = min(p_hi, q_end_pos - 1);
         if (split && is_sink && min(e_t, q_end_pos) - 1 - t > p.window) {
           const int slot_ws = gm.far ? gm.far - 1 : p.far_segs + i_t;
-          ws = p.far_ws + ((static_cast<long long>(gm.b * p.hkv + gm.hk) * p.far_slots + slot_ws) * n_sink + (t - s_t)) * 256 + half * 64;
+          ws = p.far_ws + ((static_cast<long long>(gm.b * p.hkv + gm.hk) * p.far_slots + slot_ws) * n_sink + (t - s_t)) * 256 + half * (kD / 2);
         }
         if (!kPlain && gm.far) p_lo = t + p.window + 1, p_hi = gm.far_hi;
       }
@@ -595,19 +597,19 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         pend_sp = gm.sp;
         pend_ws = ws;
         // (a far item stores nothing for a row that has no far query: the row's key tile writes it directly)
-        pend_off = valid_k && (kPlain || gm.far == 0 || ws != nullptr) ? gm.b * p.dkv_sb[gm.sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[gm.sp] + gm.hk * p.dkv_sh[gm.sp] + half * 64 : -1;
+        pend_off = valid_k && (kPlain || gm.far == 0 || ws != nullptr) ? gm.b * p.dkv_sb[gm.sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[gm.sp] + gm.hk * p.dkv_sh[gm.sp] + half * (kD / 2) : -1;
         gbase += n_iter;
         ++nk;
       } else if (valid_k) {
         // no query of this call sees the tile: zero gradients
         const int sp = gm.sp;
-        const long long off = gm.b * p.dkv_sb[sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[sp] + gm.hk * p.dkv_sh[sp] + half * 64;
+        const long long off = gm.b * p.dkv_sb[sp] + static_cast<long long>(gm.key0 + row) * p.dkv_st[sp] + gm.hk * p.dkv_sh[sp] + half * (kD / 2);
         const bool f32 = !kPlain && (p.grad_fp32[sp] != 0 || ws != nullptr);
         const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll 1
         for (int which = 0; which < 2; ++which) {
           void* base = which == 0 ? p.dk[sp] : p.dv[sp];
-          const int n32 = f32 ? 8 : 4;  // 32-byte pieces of this thread's 64 columns
+          const int n32 = f32 ? kD / 16 : kD / 32;  // 32-byte pieces of this thread's columns
           uint8_t* dst = f32 ? reinterpret_cast<uint8_t*>(static_cast<float*>(base) + off) : reinterpret_cast<uint8_t*>(static_cast<uint16_t*>(base) + off);
           if (!kPlain && ws != nullptr) dst = reinterpret_cast<uint8_t*>(ws + which * 128);
 #pragma unroll 1
@@ -629,7 +631,8 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
 }
 
 // Adds up the parts of the sink rows' gradients: the windowed part and the far segments of the row's sequence,
-// in a fixed order.  One block per (batch row, KV head, sequence, sink row); thread = (dK or dV, column).
+// in a fixed order.  One block per (batch row, KV head, sequence, sink row); thread = (dK or dV, column).  A row of
+// partial sums is 2 x 128 floats whatever the head's width.
 // A handful of 512-byte rows per block: latency, 4 us where it replaced a serial chain of milliseconds.
 template <bool kBf16>
 __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ BwdKernelParams p) {
@@ -642,7 +645,9 @@ __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ B
   int sp = 0;
   while (sp < p.n_spans && (t < p.span_pos[sp] || t >= p.span_pos[sp] + p.span_len[sp])) ++sp;
   if (sp == p.n_spans) return;
-  const float* ws = p.far_ws + (static_cast<long long>(b * p.hkv + hk) * p.far_slots * p.n_sink + r) * 256 + threadIdx.x;
+  const int width = blockDim.x >> 1;
+  const int which = threadIdx.x >= width ? 1 : 0, c = threadIdx.x - which * width;
+  const float* ws = p.far_ws + (static_cast<long long>(b * p.hkv + hk) * p.far_slots * p.n_sink + r) * 256 + which * 128 + c;
   const long long slot = p.n_sink * 256LL;
   float sum = ws[(p.far_segs + i) * slot];
   // chunk boundaries below the sequence's start / its end (a start comes first on a tie): the segments are
@@ -655,7 +660,6 @@ __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ B
     far_range(p, i, j, s, e, q_lo, q_hi);
     if (q_lo <= q_hi) sum += ws[(i + j) * slot];
   }
-  const int which = threadIdx.x >> 7, c = threadIdx.x & 127;
   const long long off = b * p.dkv_sb[sp] + static_cast<long long>(t - p.span_pos[sp]) * p.dkv_st[sp] + hk * p.dkv_sh[sp] + c;
   void* base = which == 0 ? p.dk[sp] : p.dv[sp];
   if (p.grad_fp32[sp]) static_cast<float*>(base)[off] = sum;
@@ -673,13 +677,15 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool e
     return RSWA_E_ARG;
   }
   const bool plain = kp.n_spans == 1 && kp.cu == nullptr && kp.n_sink == 0 && kp.grad_fp32[0] == 0;
-  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (plain ? 2 : 0);
+  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (plain ? 2 : 0) + (kp.head_dim == kNarrowHeadDim ? 4 : 0);
   using Kern = void (*)(const BwdKernelParams, int);
-  static const Kern kerns[4] = {rswa_bwd_kernel<false, false>, rswa_bwd_kernel<true, false>,
-                                rswa_bwd_kernel<false, true>, rswa_bwd_kernel<true, true>};
+  static const Kern kerns[8] = {rswa_bwd_kernel<128, false, false>, rswa_bwd_kernel<128, true, false>,
+                                rswa_bwd_kernel<128, false, true>,  rswa_bwd_kernel<128, true, true>,
+                                rswa_bwd_kernel<64, false, false>,  rswa_bwd_kernel<64, true, false>,
+                                rswa_bwd_kernel<64, false, true>,   rswa_bwd_kernel<64, true, true>};
   const Kern kern = kerns[variant];
   // (the attribute is a property of the function on a device: set once per kernel variant and device)
-  static bool attr_set[4][64] = {{false}};
+  static bool attr_set[8][64] = {{false}};
   int dev_id = 0;
   cudaError_t e = cudaGetDevice(&dev_id);
   if (e == cudaSuccess && (dev_id < 0 || dev_id >= 64 || !attr_set[variant][dev_id])) {
@@ -706,8 +712,8 @@ int launch_sink_sum(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
   if (kp.far_segs > 0) {
     const int n_seq = kp.cu == nullptr ? 1 : kp.n_seqs + 1;
     const dim3 grid(static_cast<unsigned>(n_seq * kp.n_sink), static_cast<unsigned>(kp.hkv), static_cast<unsigned>(kp.batch));
-    if (dtype == RSWA_DTYPE_BF16) sink_sum_kernel<true><<<grid, 256, 0, stream>>>(kp);
-    else sink_sum_kernel<false><<<grid, 256, 0, stream>>>(kp);
+    if (dtype == RSWA_DTYPE_BF16) sink_sum_kernel<true><<<grid, 2 * kp.head_dim, 0, stream>>>(kp);
+    else sink_sum_kernel<false><<<grid, 2 * kp.head_dim, 0, stream>>>(kp);
     count_launches(1);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

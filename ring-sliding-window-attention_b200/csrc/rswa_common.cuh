@@ -10,6 +10,12 @@ namespace rswa {
 
 constexpr int kTile = RSWA_TILE;       // rows of a query tile and of a key tile
 constexpr int kHeadDim = 128;
+// Heads of 64 elements have kernels of their own (the template argument kD): a tile is one TMA box instead of two,
+// the products that contract over the head dimension take half as many instructions, the others are half as wide.
+// Shared and tensor memory keep the 128-wide layout, half of each tile unused: neither leaves room for a second CTA
+// per SM either way (the registers do not).  Training step, zero-padded to 128 by the host -> these kernels:
+// 4 x 4096 tokens, 16 heads, window 512: 767 -> 342 us; 1024 tokens, 4 heads, window 128: 320 -> 91 us.
+constexpr int kNarrowHeadDim = 64;
 constexpr int kBoxBytes = 16384;       // one TMA box: 128 rows x 64 x 16-bit, 128-byte swizzle
 constexpr int kTileBytes = 2 * kBoxBytes;
 constexpr int kMaxEntries = 2 * RSWA_MAX_SPANS;
@@ -29,7 +35,7 @@ struct FwdKernelParams {
   int span_pos[RSWA_MAX_SPANS];
   int span_len[RSWA_MAX_SPANS];
   int n_spans;
-  int batch, q_len, hq, hkv;
+  int batch, q_len, hq, hkv, head_dim;
   int q_pos_start, window, n_sink;
   float scale_log2;  // softmax_scale * log2(e)
   const int* cu;
@@ -57,7 +63,7 @@ struct BwdKernelParams {
   long long dkv_sb[RSWA_MAX_SPANS], dkv_st[RSWA_MAX_SPANS], dkv_sh[RSWA_MAX_SPANS];
   int grad_fp32[RSWA_MAX_SPANS];
   int n_spans;
-  int batch, q_len, hq, hkv;
+  int batch, q_len, hq, hkv, head_dim;
   int q_pos_start, window, n_sink;
   float scale_log2;
   float scale;
@@ -180,11 +186,11 @@ __device__ __forceinline__ int far_sequence(const BwdKernelParams& p, int e) {
 
 // host side -------------------------------------------------------------------------------
 void set_error(const char* fmt, ...);
-// 4-D map over a [batch, tokens, heads, 128] 16-bit tensor (strides in elements), box = 64
+// 4-D map over a [batch, tokens, heads, head_dim] 16-bit tensor (strides in elements), box = 64
 // elements x 1 head x 128 tokens x 1 batch, 128-byte swizzle, zero fill out of bounds.
-int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int tokens, int heads,
+int make_tile_map(CUtensorMap* map, const void* base, int dtype, int batch, int tokens, int heads, int head_dim,
                   long long sb, long long st, long long sh);
-int check_geom(const rswa_geom_t& g, bool need_grads);
+int check_geom(const rswa_geom_t& g, bool need_grads, int head_dim = kHeadDim);
 int* status_mirror(const int* status);  // the mirror registered for a status word, or null
 void count_launches(int n);             // kernels of this library launched (rswa_launch_count)
 int sm_count();  // SMs of the current device (cached per device)

@@ -86,9 +86,11 @@ __device__ __forceinline__ DqItem dq_item(const BwdKernelParams& p, int n_q_tile
 // kPlain: one KV span, no packed sequences, no sink tokens (the plain sliding window of one GPU).  The
 // SM's instruction cache holds 32 KB and this kernel's five roles together execute more than that per
 // work item, so what such a call cannot need is compiled out of its variant.
-template <bool kBf16, bool kPlain>
+// kD: width of a head, 128 or 64.
+template <int kD, bool kBf16, bool kPlain>
 __global__ void __launch_bounds__(kDqThreads, 1)
 rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_items) {
+  constexpr uint32_t kLoadBytes = kD / 64 * kBoxBytes;  // what a tile holds (its slots in shared memory are kTileBytes apart)
   const int* const cu_seq = kPlain ? nullptr : p.cu;
   const int n_seqs = kPlain ? 0 : p.n_seqs;
   const int n_spans = kPlain ? 1 : p.n_spans;
@@ -187,27 +189,27 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
           cursor_begin<kTile>(geom, p.span_pos, p.span_len, c);
           // Q may be replaced once the last S product of the previous item has read it
           if (ic > 0 && !mbar_wait<200>(&ctl->q_free, (ic - 1) & 1, err, kErrWaitProducer)) break;
-          mbar_expect_tx(&ctl->q_full, kTileBytes);
+          mbar_expect_tx(&ctl->q_full, kLoadBytes);
           tma_load_4d(sQ, &p.q_map, &ctl->q_full, 0, w.h, w.row0, w.b);
-          tma_load_4d(sQ + kBoxBytes, &p.q_map, &ctl->q_full, 64, w.h, w.row0, w.b);
+          if (kD > 64) tma_load_4d(sQ + kBoxBytes, &p.q_map, &ctl->q_full, 64, w.h, w.row0, w.b);
         }
         const int sk = kc % kDqKStages, sv = kc & 1;
         if (kc >= kDqKStages && !mbar_wait<200>(&ctl->k_free[sk], ((kc / kDqKStages) - 1) & 1, err, kErrWaitProducer)) break;
-        mbar_expect_tx(&ctl->k_full[sk], kTileBytes);
+        mbar_expect_tx(&ctl->k_full[sk], kLoadBytes);
         tma_load_4d(sK + sk * kTileBytes, &p.k_map[c.span], &ctl->k_full[sk], 0, w.hk, c.tok, w.b);
-        tma_load_4d(sK + sk * kTileBytes + kBoxBytes, &p.k_map[c.span], &ctl->k_full[sk], 64, w.hk, c.tok, w.b);
+        if (kD > 64) tma_load_4d(sK + sk * kTileBytes + kBoxBytes, &p.k_map[c.span], &ctl->k_full[sk], 64, w.hk, c.tok, w.b);
         if (j == 0) {
           // dO likewise, after the last dP product of the previous item
           if (ic > 0 && !mbar_wait<200>(&ctl->do_free, (ic - 1) & 1, err, kErrWaitProducer)) break;
           ++ic;
-          mbar_expect_tx(&ctl->do_full, kTileBytes);
+          mbar_expect_tx(&ctl->do_full, kLoadBytes);
           tma_load_4d(sDO, &p.do_map, &ctl->do_full, 0, w.h, w.row0, w.b);
-          tma_load_4d(sDO + kBoxBytes, &p.do_map, &ctl->do_full, 64, w.h, w.row0, w.b);
+          if (kD > 64) tma_load_4d(sDO + kBoxBytes, &p.do_map, &ctl->do_full, 64, w.h, w.row0, w.b);
         }
         if (kc >= 2 && !mbar_wait<200>(&ctl->v_free[sv], ((kc >> 1) - 1) & 1, err, kErrWaitProducer)) break;
-        mbar_expect_tx(&ctl->v_full[sv], kTileBytes);
+        mbar_expect_tx(&ctl->v_full[sv], kLoadBytes);
         tma_load_4d(sV + sv * kTileBytes, &p.v_map[c.span], &ctl->v_full[sv], 0, w.hk, c.tok, w.b);
-        tma_load_4d(sV + sv * kTileBytes + kBoxBytes, &p.v_map[c.span], &ctl->v_full[sv], 64, w.hk, c.tok, w.b);
+        if (kD > 64) tma_load_4d(sV + sv * kTileBytes + kBoxBytes, &p.v_map[c.span], &ctl->v_full[sv], 64, w.hk, c.tok, w.b);
         ++j;
         ++kc;
         cursor_next<kTile>(geom, p.span_pos, p.span_len, c, j < n_tiles);
@@ -218,9 +220,9 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
       constexpr uint32_t kTile16 = kTileBytes >> 4;
       const uint64_t dQd = smem_desc_sw128(smem_u32(sQ), 16, 1024);
       const uint64_t dKk = smem_desc_sw128(smem_u32(sK), 16, 1024);  // K as K-major B operand
-      uint64_t dqa[8];  // the A operands never change: Q has one buffer
+      uint64_t dqa[kD / 16];  // the A operands never change: Q has one buffer
 #pragma unroll
-      for (int k = 0; k < 8; ++k) dqa[k] = dQd + ((((k >> 2) * kBoxBytes + (k & 3) * 32)) >> 4);
+      for (int k = 0; k < kD / 16; ++k) dqa[k] = dQd + ((((k >> 2) * kBoxBytes + (k & 3) * 32)) >> 4);
       bool ok = true;
       int n = 0, kc = 0, ic = 0;  // kc: key tiles of earlier items = running index of this item's tile 0
       for (;; ++n) {
@@ -233,13 +235,13 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
           for (int j = 0; j < n_tiles && ok; ++j) {
             const int g = kc + j;
             const int sk = g % kDqKStages;
-            // every operand of the eight instructions is in a register BEFORE the waits: what this
+            // every operand of the instructions is in a register BEFORE the waits: what this
             // thread executes between the last barrier and the last instruction is on the chain that
             // bounds the kernel, and it gets an instruction through only every few cycles
-            uint64_t db[8];
+            uint64_t db[kD / 16];
             const uint32_t td = tmem + 128 * (g & 1);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < kD / 16; ++k) {
               db[k] = dKk + sk * kTile16 + ((((k >> 2) * kBoxBytes + (k & 3) * 32)) >> 4);
               asm volatile("" : "+l"(db[k]));
             }
@@ -250,7 +252,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
             DQ_TRC(true, g, 0);
             tc_fence_after();
 #pragma unroll
-            for (int k = 0; k < 8; ++k) mma_ss(td, dqa[k], db[k], id_kk, k > 0 ? 1u : 0u);
+            for (int k = 0; k < kD / 16; ++k) mma_ss(td, dqa[k], db[k], id_kk, k > 0 ? 1u : 0u);
             DQ_TRC(true, g, 1);
             mma_commit(&ctl->s_ready[g & 1]);
             if (j + 1 == n_tiles) mma_commit(&ctl->q_free);  // that was the item's last read of Q
@@ -262,7 +264,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
       }
     } else if (warp == 3 && elect_one()) {
       // ------------------------------------------------------------------ MMA issuer 3: dQ += dS K
-      constexpr uint32_t id_tn = idesc_f16(128, 128, kBf16 ? 1 : 0, 0, 1);
+      constexpr uint32_t id_tn = idesc_f16(128, kD, kBf16 ? 1 : 0, 0, 1);
       constexpr uint32_t kTile16 = kTileBytes >> 4;
       const uint64_t dKm = smem_desc_sw128(smem_u32(sK), kBoxBytes, 1024);  // K as MN-major B operand
       bool ok = true;
@@ -329,7 +331,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
             tc_fence_after();
             const uint64_t dVs = dVk + sv * kTile16;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < kD / 16; ++k) {
               const uint32_t off = ((k >> 2) * kBoxBytes + (k & 3) * 32) >> 4;
               mma_ss(tDP, dDO + off, dVs + off, id_kk, k > 0 ? 1u : 0u);
             }
@@ -367,7 +369,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
     // An item's dQ is read out of tensor memory and stored only after the first exponentials of the
     // NEXT item: its last product is still running when its last dS has been handed over, and waiting
     // for it right there left every compute warp idle.
-    uint16_t* pend_row = nullptr;  // where this thread's 32 values of the pending item go (null: row does not exist)
+    uint16_t* pend_row = nullptr;  // where this thread's kD / 4 values of the pending item go (null: row does not exist)
     bool pend = false;
     int pend_ic = 0;
     auto drain = [&]() -> bool {
@@ -375,8 +377,9 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
       k = __all_sync(0xffffffffu, k);
       if (!k) return false;
       tc_fence_after();
-      uint32_t r[32];
-      tmem_ld32(tDQ + lane_off + part * 32, r);
+      uint32_t r[kD / 4];
+      if constexpr (kD == 128) tmem_ld32(tDQ + lane_off + part * 32, r);
+      else tmem_ld16(tDQ + lane_off + part * 16, r);
       tmem_ld_wait();
       // the accumulator is released as soon as it is in registers
       tc_fence_before();
@@ -385,7 +388,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
       if (pend_row != nullptr) {
         // (32-byte stores: whole sectors, half as many requests as 16-byte ones)
 #pragma unroll
-        for (int v = 0; v < 2; ++v) {
+        for (int v = 0; v < kD / 64; ++v) {
           uint32_t o[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -513,7 +516,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
         if (it_nx >= 0) row_stats(it_nx, lse2_nx, delta_nx);
       }
       uint16_t* drow = reinterpret_cast<uint16_t*>(p.dq) + w.b * p.dq_sb +
-                       static_cast<long long>(w.row0 + row) * p.dq_st + w.h * p.dq_sh + part * 32;
+                       static_cast<long long>(w.row0 + row) * p.dq_st + w.h * p.dq_sh + part * (kD / 4);
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->geom_free[slot]);  // (the list is not needed any more)
       if (n_tiles > 0) {
@@ -527,7 +530,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
         // no key of the given spans is visible to this query tile
         uint4* dst = reinterpret_cast<uint4*>(drow);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) dst[v] = make_uint4(0, 0, 0, 0);
+        for (int v = 0; v < kD / 32; ++v) dst[v] = make_uint4(0, 0, 0, 0);
       }
     }
     if (ok && pend) ok = drain();
@@ -555,13 +558,15 @@ int launch_dq(const BwdKernelParams& kp, int dtype, bool early, cudaStream_t str
     return RSWA_E_ARG;
   }
   const bool plain = kp.n_spans == 1 && kp.cu == nullptr && kp.n_sink == 0;
-  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (plain ? 2 : 0);
+  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (plain ? 2 : 0) + (kp.head_dim == kNarrowHeadDim ? 4 : 0);
   using Kern = void (*)(const BwdKernelParams, int, int);
-  static const Kern kerns[4] = {rswa_dq_kernel<false, false>, rswa_dq_kernel<true, false>,
-                                rswa_dq_kernel<false, true>, rswa_dq_kernel<true, true>};
+  static const Kern kerns[8] = {rswa_dq_kernel<128, false, false>, rswa_dq_kernel<128, true, false>,
+                                rswa_dq_kernel<128, false, true>,  rswa_dq_kernel<128, true, true>,
+                                rswa_dq_kernel<64, false, false>,  rswa_dq_kernel<64, true, false>,
+                                rswa_dq_kernel<64, false, true>,   rswa_dq_kernel<64, true, true>};
   const Kern kern = kerns[variant];
   // (the attribute is a property of the function on a device: set once per kernel variant and device)
-  static bool attr_set[4][64] = {{false}};
+  static bool attr_set[8][64] = {{false}};
   int dev_id = 0;
   cudaError_t e = cudaGetDevice(&dev_id);
   if (e == cudaSuccess && (dev_id < 0 || dev_id >= 64 || !attr_set[variant][dev_id])) {

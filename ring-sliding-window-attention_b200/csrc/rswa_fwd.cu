@@ -110,9 +110,11 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int n_bloc
 // kCarry:  out / lse hold a partial result that the call continues;
 // kSimple: one KV span, no packed sequences, no sink tokens (the plain sliding window of one GPU, and
 //          the tiles of a ring call that need no halo): the geometry collapses to a few lines.
-template <bool kBf16, bool kCarry, bool kSimple>
+// kD:      width of a head, 128 or 64.
+template <int kD, bool kBf16, bool kCarry, bool kSimple>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_items) {
+  constexpr uint32_t kLoadBytes = kD / 64 * kBoxBytes;  // what a tile holds (its slots in shared memory are kTileBytes apart)
   const int* const cu_seq = kSimple ? nullptr : p.cu;
   const int n_seqs = kSimple ? 0 : p.n_seqs;
   const int n_spans = kSimple ? 1 : p.n_spans;
@@ -214,13 +216,13 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
         const int st = u & 1;
         if (u >= kUnits && !mbar_wait<100>(&ctl->kv_free[st], ((u >> 1) - 1) & 1, err, kErrWaitProducer)) break;
         ctl->unit_flags[u & 7] = flags;
-        const uint32_t bytes = (has_k ? kTileBytes : 0) + (pend ? kTileBytes : 0);
+        const uint32_t bytes = (has_k ? kLoadBytes : 0) + (pend ? kLoadBytes : 0);
         if (bytes > 0) mbar_expect_tx(&ctl->kv_full[st], bytes);  // (release: the flags are visible to whoever sees the unit)
         else mbar_arrive(&ctl->kv_full[st]);
         uint8_t* dst = sU + st * 2 * kTileBytes;
         if (pend) {
           tma_load_4d(dst + kTileBytes, &p.v_map[pv_span], &ctl->kv_full[st], 0, pv_hk, pv_tok, pv_b);
-          tma_load_4d(dst + kTileBytes + kBoxBytes, &p.v_map[pv_span], &ctl->kv_full[st], 64, pv_hk, pv_tok, pv_b);
+          if (kD > 64) tma_load_4d(dst + kTileBytes + kBoxBytes, &p.v_map[pv_span], &ctl->kv_full[st], 64, pv_hk, pv_tok, pv_b);
         }
         ++u;
         if (!has_k) {
@@ -230,7 +232,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
         }
         RSWA_TRC(fwd, n == RSWA_TRACE_ITEM && j < 32, j * 32 + 16);
         tma_load_4d(dst, &p.k_map[c.span], &ctl->kv_full[st], 0, w.hk, c.tok, w.b);
-        tma_load_4d(dst + kBoxBytes, &p.k_map[c.span], &ctl->kv_full[st], 64, w.hk, c.tok, w.b);
+        if (kD > 64) tma_load_4d(dst + kBoxBytes, &p.k_map[c.span], &ctl->kv_full[st], 64, w.hk, c.tok, w.b);
         pend = true;
         pv_span = c.span, pv_tok = c.tok, pv_hk = w.hk, pv_b = w.b;
         if (j == 0) {
@@ -238,11 +240,12 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
           if (ic > 0 && !mbar_wait<100>(&ctl->q_free, (ic - 1) & 1, err, kErrWaitProducer)) break;
           ++ic;
           const int n_q = geom->n_valid[1] > 0 ? 2 : 1;
-          mbar_expect_tx(&ctl->q_full, n_q * kTileBytes);
+          constexpr int kBoxes = kD / 64;
+          mbar_expect_tx(&ctl->q_full, n_q * kLoadBytes);
 #pragma unroll 1
-          for (int i = 0; i < 2 * n_q; ++i) {
-            tma_load_4d(sQ + (i >> 1) * kTileBytes + (i & 1) * kBoxBytes, &p.q_map, &ctl->q_full, (i & 1) * 64, w.h,
-                        (w.tile0 + (i >> 1)) * kTile, w.b);
+          for (int i = 0; i < kBoxes * n_q; ++i) {
+            tma_load_4d(sQ + (i / kBoxes) * kTileBytes + (i % kBoxes) * kBoxBytes, &p.q_map, &ctl->q_full, (i % kBoxes) * 64, w.h,
+                        (w.tile0 + i / kBoxes) * kTile, w.b);
           }
         }
         ++j;
@@ -257,7 +260,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
       // comes from the producer's flags), one barrier per unit of loads, no warp votes.
       if (elect_one() && n_work > 0) {
         constexpr uint32_t idesc_qk = idesc_f16(128, 128, kBf16 ? 1 : 0, 0, 0);
-        constexpr uint32_t idesc_pv = idesc_f16(128, 128, kBf16 ? 1 : 0, 0, 1);
+        constexpr uint32_t idesc_pv = idesc_f16(128, kD, kBf16 ? 1 : 0, 0, 1);
         // descriptors are built once; per stage / k-step only their address field moves (16-byte units)
         constexpr uint32_t kTile16 = kTileBytes >> 4;
         const uint64_t dQ = smem_desc_sw128(smem_u32(sQ), 16, 1024);
@@ -320,7 +323,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
               }
               // overwrites P_w of the previous key tile: ordered behind the product just issued
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
+              for (int k = 0; k < kD / 16; ++k) {
                 const uint32_t off = ((k >> 2) * kBoxBytes + (k & 3) * 32) >> 4;
                 mma_ss(tSw, dQ + w * kTile16 + off, dKs + off, idesc_qk, k > 0 ? 1u : 0u);
               }
@@ -406,7 +409,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
             l_sum = had ? 1.f : 0.f;
             const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.out) + orow);
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < kD / 32; ++c) {
               uint32_t o[32];
 #pragma unroll
               for (int v4 = 0; v4 < 4; ++v4) {
@@ -507,7 +510,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
             tc_fence_after();
             l_sum *= alpha;
 #pragma unroll 1
-            for (int c = 0; c < 8; ++c) {  // (in small pieces: the S row occupies most of the registers)
+            for (int c = 0; c < kD / 16; ++c) {  // (in small pieces: the S row occupies most of the registers)
               uint32_t o[16];
               tmem_ld16(tO + c * 16, o);
               tmem_ld_wait();
@@ -575,9 +578,9 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
         if (!ok) break;
         RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM, 1925 + 4 * w);
         tc_fence_after();
-        uint32_t o[128];
+        uint32_t o[kD];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(tO + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[c * 32]));
+        for (int c = 0; c < kD / 32; ++c) tmem_ld32(tO + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[c * 32]));
         tmem_ld_wait();
         // the accumulator is in registers: the next item's first product may overwrite it
         tc_fence_before();
@@ -591,7 +594,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
                           static_cast<long long>(tile_row0 + quad * 32) * p.o_st + wi.h * p.o_sh;
         const int ch = lane & 7;
 #pragma unroll 1  // (one copy of the code; the second half of the row moves down in the registers)
-        for (int pass = 0; pass < 2; ++pass) {
+        for (int pass = 0; pass < kD / 64; ++pass) {
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
             const int e0 = v * 8;
@@ -611,7 +614,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
           }
           __syncwarp();  // the staging rows are rewritten by the next pass / item
 #pragma unroll
-          for (int i = 0; i < 64; ++i) o[i] = o[64 + i];
+          for (int i = 64; i < kD; ++i) o[i - 64] = o[i];
         }
       } else if (valid && !kCarry) {
         // no key of the given spans is visible to this query tile: zero rows (a carried-in partial
@@ -619,7 +622,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
         uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + wi.b * p.o_sb +
                                               static_cast<long long>(tile_row0 + row) * p.o_st + wi.h * p.o_sh);
 #pragma unroll
-        for (int v = 0; v < 16; ++v) dst[v] = make_uint4(0, 0, 0, 0);
+        for (int v = 0; v < kD / 8; ++v) dst[v] = make_uint4(0, 0, 0, 0);
       }
       if (valid && (n_done > 0 || !kCarry)) {
         p.lse[wi.b * p.l_sb + wi.h * p.l_sh + tile_row0 + row] =
@@ -653,15 +656,18 @@ int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream) {
     return RSWA_E_ARG;
   }
   const bool simple = kp.n_spans == 1 && kp.cu == nullptr && kp.n_sink == 0;
-  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (kp.carry ? 2 : 0) + (simple ? 4 : 0);
+  const bool narrow = kp.head_dim == kNarrowHeadDim;  // (nothing to carry in then, see the API)
+  const int variant = (dtype == RSWA_DTYPE_BF16 ? 1 : 0) + (narrow ? 8 + (simple ? 2 : 0) : (kp.carry ? 2 : 0) + (simple ? 4 : 0));
   using Kern = void (*)(const FwdKernelParams, int, int);
-  static const Kern kerns[8] = {rswa_fwd_kernel<false, false, false>, rswa_fwd_kernel<true, false, false>,
-                                rswa_fwd_kernel<false, true, false>,  rswa_fwd_kernel<true, true, false>,
-                                rswa_fwd_kernel<false, false, true>,  rswa_fwd_kernel<true, false, true>,
-                                rswa_fwd_kernel<false, true, true>,   rswa_fwd_kernel<true, true, true>};
+  static const Kern kerns[12] = {rswa_fwd_kernel<128, false, false, false>, rswa_fwd_kernel<128, true, false, false>,
+                                 rswa_fwd_kernel<128, false, true, false>,  rswa_fwd_kernel<128, true, true, false>,
+                                 rswa_fwd_kernel<128, false, false, true>,  rswa_fwd_kernel<128, true, false, true>,
+                                 rswa_fwd_kernel<128, false, true, true>,   rswa_fwd_kernel<128, true, true, true>,
+                                 rswa_fwd_kernel<64, false, false, false>,  rswa_fwd_kernel<64, true, false, false>,
+                                 rswa_fwd_kernel<64, false, false, true>,   rswa_fwd_kernel<64, true, false, true>};
   const Kern kern = kerns[variant];
   // (the attribute is a property of the function on a device: set once per kernel variant and device)
-  static bool attr_set[8][64] = {{false}};
+  static bool attr_set[12][64] = {{false}};
   int dev_id = 0;
   cudaError_t e = cudaGetDevice(&dev_id);
   if (e == cudaSuccess && (dev_id < 0 || dev_id >= 64 || !attr_set[variant][dev_id])) {

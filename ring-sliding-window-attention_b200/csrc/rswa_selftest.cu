@@ -131,9 +131,9 @@ extern "C" int rswa_selftest_mma(int32_t mode, const void* a, const void* b, flo
     return RSWA_E_ARG;
   }
   CUtensorMap am, bm;
-  int rc = make_tile_map(&am, a, RSWA_DTYPE_BF16, 1, 128, 1, 128 * 128, 128, 128);
+  int rc = make_tile_map(&am, a, RSWA_DTYPE_BF16, 1, 128, 1, kHeadDim, 128 * 128, 128, 128);
   if (rc) return rc;
-  rc = make_tile_map(&bm, b, RSWA_DTYPE_BF16, 1, 128, 1, 128 * 128, 128, 128);
+  rc = make_tile_map(&bm, b, RSWA_DTYPE_BF16, 1, 128, 1, kHeadDim, 128 * 128, 128, 128);
   if (rc) return rc;
   const int smem = 2 * kTileBytes + 1024 + 256;
   cudaError_t e = cudaFuncSetAttribute(selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -25,7 +25,7 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int64_t kMaxHeadDim = 128;
+constexpr int64_t kHeadDim = 128, kNarrowHeadDim = 64;  // the widths that have kernels
 // per device: the status word the kernels raise and its host mirror (ring_swa/_kernels.py owns both)
 int32_t* g_status[kMaxDevices] = {nullptr};
 const volatile int32_t* g_mirror[kMaxDevices] = {nullptr};
@@ -107,7 +107,8 @@ at::Tensor forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
   p.lse = lse.data_ptr<float>();
   p.lse_stride_b = d.heads * d.tokens, p.lse_stride_h = d.tokens;
   p.status = g_status[q.get_device()];
-  check(rswa_fwd(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_fwd");
+  const auto call = q.size(-1) == kNarrowHeadDim ? rswa_fwd_d64 : rswa_fwd;
+  check(call(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_fwd");
   return out;
 }
 
@@ -135,7 +136,7 @@ class SwaFunction : public torch::autograd::Function<SwaFunction> {
     at::Tensor dk = at::empty(k.sizes(), k.options()), dv = at::empty(k.sizes(), k.options());
     const Dims d = dims_of(q);
     const int64_t hkv = dims_of(k).heads;
-    int64_t ws_bytes = rswa_bwd_workspace_bytes(d.batch, d.tokens, d.heads, q.size(-1));
+    int64_t ws_bytes = rswa_bwd_workspace_bytes(d.batch, d.tokens, d.heads, kHeadDim);
     if (c.n_sink > 0) ws_bytes += rswa_bwd_sink_workspace_bytes(d.batch, d.tokens, hkv, c.window, c.n_sink, cu.defined() ? cu.numel() - 1 : 0);
     at::Tensor ws = at::empty({ws_bytes}, q.options().dtype(at::kByte));
 
@@ -162,7 +163,8 @@ class SwaFunction : public torch::autograd::Function<SwaFunction> {
     p.workspace_bytes = ws_bytes;
     p.flags = RSWA_BWD_INIT | RSWA_BWD_FINISH;
     p.status = g_status[q.get_device()];
-    check(rswa_bwd(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_bwd");
+    const auto call = q.size(-1) == kNarrowHeadDim ? rswa_bwd_d64 : rswa_bwd;
+    check(call(&p, c10::cuda::getCurrentCUDAStream(q.get_device()).stream()), "rswa_bwd");
     return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
@@ -176,7 +178,7 @@ bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, con
   if (dev < 0 || dev >= kMaxDevices || g_mirror[dev] == nullptr || *g_mirror[dev] != 0) return false;
   if (dev != c10::cuda::current_device()) return false;
   if (q.dim() != (cu.defined() ? 3 : 4) || k.dim() != q.dim() || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return false;
-  if (q.size(-1) != kMaxHeadDim || k.size(-1) != kMaxHeadDim) return false;
+  if ((q.size(-1) != kHeadDim && q.size(-1) != kNarrowHeadDim) || k.size(-1) != q.size(-1)) return false;
   const Dims dq = dims_of(q), dk = dims_of(k);
   if (dq.batch != dk.batch || dq.tokens != dk.tokens || dq.heads % dk.heads != 0) return false;
   if (dq.batch > 0x7fffffff || dq.tokens > 0x7fffffff || dq.heads > 0x7fffffff) return false;

@@ -95,9 +95,11 @@ SYMBOLS = {
     "rswa_abi_version": (C.c_int, []),
     "rswa_last_error": (C.c_char_p, []),
     "rswa_fwd": (C.c_int, [C.POINTER(FwdParams), C.c_void_p]),
+    "rswa_fwd_d64": (C.c_int, [C.POINTER(FwdParams), C.c_void_p]),
     "rswa_bwd_workspace_bytes": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "rswa_bwd_sink_workspace_bytes": (C.c_int64, [C.c_int32] * 6),
     "rswa_bwd": (C.c_int, [C.POINTER(BwdParams), C.c_void_p]),
+    "rswa_bwd_d64": (C.c_int, [C.POINTER(BwdParams), C.c_void_p]),
     "rswa_bwd_noalloc": (C.c_int, [C.POINTER(BwdParams), C.c_void_p]),
     "rswa_noalloc_scratch_bytes": (C.c_int64, []),
     "rswa_merge": (C.c_int, [C.POINTER(MergeParams), C.c_void_p]),

@@ -413,8 +413,8 @@ def attention(q, k, v, window_size: int, n_sink: int, softmax_scale: Optional[fl
     if softmax_scale is None:
         softmax_scale = head_dim ** (-0.5)
     if q.is_cuda and head_dim < K.HEAD_DIM:
-        # The kernels are built for a head dimension of 128.  Smaller ones (the reference's own local
-        # tests use 64) run on them zero-padded: the padding adds nothing to any score, the padded
+        # The kernels are built for a head dimension of 128, and of 64 for single_gpu() above.  Other ones, and
+        # 64 across several GPUs, run on the 128-wide ones zero-padded: the padding adds nothing to any score, the padded
         # output and gradient columns are zero and are cut off again -- at the price of the arithmetic
         # and traffic of a 128-wide head.  The scale keeps referring to the caller's head dimension.
         if head_dim % 8:

@@ -367,3 +367,44 @@ def test_full_size_long_window_spot_blocks():
         assert_close(f"dk[{a}:{b}]", dk[0, a:b, kh], rdk)
         assert_close(f"dv[{a}:{b}]", dv[0, a:b, kh], rdv)
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,W,n_sink,lens,dtype,fused", [
+    (1, 1, 1, 1, 0, 0, None, torch.bfloat16, False),
+    (1, 128, 2, 2, 127, 0, None, torch.bfloat16, False),
+    (2, 257, 4, 2, 128, 0, None, torch.bfloat16, True),             # one row past two tiles, strided inputs
+    (1, 1500, 8, 1, 200, 0, None, torch.float16, True),
+    (1, 1500, 4, 2, 100, 1, None, torch.bfloat16, False),           # sink gradients in segments
+    (1, 1300, 4, 2, 130, 4, [1, 127, 700, 472], torch.bfloat16, False),
+    (1, 700, 2, 1, 90, 0, [100, 1, 299, 300], torch.float16, True),
+])
+def test_64_wide_heads(B, S, Hq, Hkv, W, n_sink, lens, dtype, fused):
+    """Heads of 64 elements have kernels of their own; the tolerances are those of 128-wide heads (the sums over
+    the head dimension are half as long, the values of the same size)."""
+    import ring_swa
+    g = torch.Generator().manual_seed(S)
+    qkv = torch.randn(B, S, Hq + 2 * Hkv, 64, generator=g).to(dtype)
+    do = torch.randn(B, S, Hq, 64, generator=g).to(dtype)
+    q, k, v = qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:]
+    cu = None
+    if lens:
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+    ro, _, rdq, rdk, rdv = dense_attn_fwd_bwd(q, k, v, do, W, None, n_sink, cu)
+    x = qkv.cuda()
+    x = [x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:]]
+    kw, fn = {}, ring_swa.ring_sliding_window_attn
+    if n_sink:
+        fn = ring_swa.ring_streaming_llm_attn
+        kw["num_sink_tokens"] = n_sink
+    if lens:
+        fn = ring_swa.ring_streaming_llm_attn_varlen if n_sink else ring_swa.ring_sliding_window_attn_varlen
+        kw.update(cu_seqlens=torch.tensor(cu, dtype=torch.int32, device="cuda"), cp_size=1)
+        x = [t[0] for t in x]
+    ql, kl, vl = ((t if fused else t.contiguous()).detach().requires_grad_(True) for t in x)
+    out = fn(ql, kl, vl, W, **kw)
+    grads = torch.autograd.grad(out, (ql, kl, vl), (do[0] if lens else do).cuda())
+    ring_swa._kernels.check_device_status()
+    for name, a, b in zip(("out", "dq", "dk", "dv"), (out, *grads), (ro, rdq, rdk, rdv)):
+        assert_close(name, a, b[0] if lens else b)
