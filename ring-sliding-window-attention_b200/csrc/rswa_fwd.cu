@@ -7,7 +7,7 @@
 //
 //   S_w = Q_w K^T      tcgen05.mma, both operands in shared memory (K-major), accumulator in TMEM
 //   P_w = softmax      warp group w: one query row per thread, whole S row in registers, P written
-//                      back (16-bit) over the same TMEM columns, in two halves of 64 keys
+//                      back (16-bit) over the same TMEM columns, in two parts of 96 and 32 keys
 //   O_w += P_w V       tcgen05.mma, A = P_w from TMEM, B = V from shared memory (MN-major)
 //
 // The issue order is  O_0 += P_0 V(g), S_0 = Q_0 K(g+1)^T, O_1 += P_1 V(g), S_1 = Q_1 K(g+1)^T, ...:
@@ -54,6 +54,11 @@ constexpr int kFwdTmemCols = 512;
 constexpr int kFwdSmemTiles = 7 * kTileBytes;  // Q_0, Q_1, output staging (one tile), 2 units of {K, V}
 constexpr int kUnits = 2;
 constexpr int kSoftmaxWarps = 8;
+// k-steps of 16 keys in the first of the two parts in which P is handed over.  The product of the second part follows
+// the last exponential on the chain that bounds the kernel, so it is the short one.  Against two halves of 64 keys
+// through one rolled copy of the code (64 register moves per tile): 2 x 16384 tokens, 32/32 heads, window 1000:
+// 629 -> 615 us; 32768 tokens, 64/8 heads, window 16384: 14.10 -> 13.39 ms.
+constexpr int kPSplit = 6;
 #ifndef RSWA_FWD_POLY_EVERY
 #define RSWA_FWD_POLY_EVERY 0
 #endif
@@ -138,7 +143,7 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&ctl->s_ready[i], 1);
-      mbar_init(&ctl->p_ready[i][0], 4);  // one arrival per softmax warp and half of P
+      mbar_init(&ctl->p_ready[i][0], 4);  // one arrival per softmax warp and part of P
       mbar_init(&ctl->p_ready[i][1], 4);
       mbar_init(&ctl->pv_done[i], 1);
       mbar_init(&ctl->o_free[i], 4);
@@ -296,14 +301,14 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
               }
 #pragma unroll
               for (int half = 0; half < 2; ++half) {
-                // P arrives in two halves of 64 keys: the first half of the product runs while the
-                // second half's exponentials are still being computed
+                // P arrives in two parts: the product of the first runs while the second's exponentials are
+                // still being computed
                 ok = mbar_wait<0>(&ctl->p_ready[w][half], (pv_phase >> w) & 1u, err, kErrWaitMma);
                 if (!ok) break;
                 RSWA_TRC(fwd, u >= RSWA_TRACE_UNIT0 && u < RSWA_TRACE_UNIT0 + 32, (u - RSWA_TRACE_UNIT0) * 32 + 1 + 4 * w + half);
                 tc_fence_after();
 #pragma unroll
-                for (int k = 4 * half; k < 4 * half + 4; ++k) {
+                for (int k = half == 0 ? 0 : kPSplit; k < (half == 0 ? kPSplit : 8); ++k) {
                   mma_ts(tOw, tSw + k * 8, dVs + k * 128, idesc_pv, (k > 0 || kCarry) ? 1u : ((pv_any >> w) & 1u));
                 }
               }
@@ -470,12 +475,11 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
             }
             tmem_st_wait();
           }
-          float2 lacc = make_float2(0.f, 0.f);
-          uint32_t r[2][2][32];  // [half of the tile][chunk of 32 columns]
+          float2 lacc;
+          uint32_t r[4][32];  // chunks of 32 columns
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, r[c >> 1][c & 1]);
+          for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, r[c]);
           tmem_ld_wait();
-          // pass 1: the row maximum
           auto max_chunk = [&](const uint32_t (&x)[32]) -> float {
             float m0 = fmax3(__uint_as_float(x[0]), __uint_as_float(x[1]), __uint_as_float(x[2]));
             float m1 = fmax3(__uint_as_float(x[3]), __uint_as_float(x[4]), __uint_as_float(x[5]));
@@ -488,11 +492,27 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
             }
             return fmax3(m0, m1, fmaxf(__uint_as_float(x[30]), __uint_as_float(x[31])));
           };
-          const float mx = fmaxf(fmaxf(max_chunk(r[0][0]), max_chunk(r[0][1])), fmaxf(max_chunk(r[1][0]), max_chunk(r[1][1])));
-          RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 11 + 8 * w);
+          const float2 sl2v = make_float2(sl2, sl2);
+          float2 nmv;
+          auto exps = [&](const uint32_t (&x)[32], uint32_t dst) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const float2 y = __ffma2_rn(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), sl2v, nmv);
+              // one pair in kPolyEvery goes through the FMA pipe instead of the special-function unit,
+              // which would otherwise need as long for a tile's exponentials as the tensor cores for
+              // its two products
+              const float2 e = (kPolyEvery > 0 && ((i >> 1) % (kPolyEvery > 0 ? kPolyEvery : 1)) == (kPolyEvery - 1))
+                                   ? ex2_poly2(y) : make_float2(ex2f(y.x), ex2f(y.y));
+              lacc = __fadd2_rn(lacc, e);
+              pk[i >> 1] = pack2<kBf16>(e.x, e.y);
+            }
+            // P (16-bit) goes over the first half of the S columns, all of which are in registers by now
+            tmem_st16(dst, pk);
+          };
           // Lazy rescale: keep the old reference maximum unless the new one exceeds it by more than 2^8,
           // so that O in TMEM is only touched rarely.
-          const float mt = mx * sl2;
+          const float mt = fmaxf(fmaxf(max_chunk(r[0]), max_chunk(r[1])), fmaxf(max_chunk(r[2]), max_chunk(r[3]))) * sl2;
           float alpha = 1.f;
           const bool grow = mt > m_ref + 8.f;
           if (grow) {
@@ -520,42 +540,27 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
             }
             tmem_st_wait();
           }
-          RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 12 + 8 * w);
           const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;  // (a row that has seen no key yet)
-          const float2 sl2v = make_float2(sl2, sl2), nmv = make_float2(-m_use, -m_use);
-          // pass 2: exponentials.  The two halves of the tile go through ONE copy of the code (the second
-          // half then moves into the first half's registers: 64 moves, against an instruction stream
-          // twice as long).
-#pragma unroll 1
-          for (int half = 0; half < 2; ++half) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              uint32_t pk[16];
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[0][c][i]), __uint_as_float(r[0][c][i + 1])), sl2v, nmv);
-                // one pair in kPolyEvery goes through the FMA pipe instead of the special-function unit,
-                // which would otherwise need as long for a tile's exponentials as the tensor cores for
-                // its two products
-                const float2 e = (kPolyEvery > 0 && ((i >> 1) % (kPolyEvery > 0 ? kPolyEvery : 1)) == (kPolyEvery - 1))
-                                     ? ex2_poly2(x) : make_float2(ex2f(x.x), ex2f(x.y));
-                lacc = __fadd2_rn(lacc, e);
-                pk[i >> 1] = pack2<kBf16>(e.x, e.y);
-              }
-              // P (16-bit) goes over the first half of the S columns, all of which are in registers by now
-              tmem_st16(tS + half * 32 + c * 16, pk);
-            }
-            // a half of P (64 keys) is complete: its share of O_w += P_w V may start
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ctl->p_ready[w][half]);
-            RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 13 + 8 * w + half);
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[0][c][i] = r[1][c][i];
-          }
+          nmv = make_float2(-m_use, -m_use);
+          lacc = make_float2(0.f, 0.f);
+          exps(r[0], tS);
+          exps(r[1], tS + 16);
+          if (!ok) break;
+          RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 12 + 8 * w);
+          // The first kPSplit k-steps of P (96 keys) are handed over when they are complete, so that their share of
+          // O_w += P_w V runs while the last 32 exponentials of the row are computed.
+          exps(r[2], tS + 32);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_ready[w][0]);
+          RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 13 + 8 * w);
+          exps(r[3], tS + 48);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->p_ready[w][1]);
+          RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 14 + 8 * w);
           l_sum += lacc.x + lacc.y;
           ++n_done;
           ++n_tot;
