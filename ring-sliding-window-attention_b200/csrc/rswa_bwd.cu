@@ -177,15 +177,16 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         int sp = 0, key0, n_valid_k, t0, q_lo, q_hi, far = 0;
         if (!kPlain && idx < p.far_segs * n_spans) {
           // The queries of one segment beyond the window of the sink tokens of their sequence: a tile that
-          // starts at the first of those this span holds (a TMA load may start at any token); the rows
-          // behind them are masked.
+          // starts at the first of those this span holds (a TMA load may start at any token).  Its rows end
+          // with the sink tokens and with the sequence: in a sequence shorter than n_sink the next rows are sink
+          // tokens of the NEXT one, whose partial sums would go to the slots of this one's.
           const int e = idx / n_spans;
           sp = idx % n_spans;
           const int i = far_sequence(p, e);
           int s_p, e_p;
           far_range(p, i, e - i, s_p, e_p, q_lo, q_hi);
           t0 = max(s_p, p.span_pos[sp]);
-          n_valid_k = min(s_p + n_sink, p.span_pos[sp] + p.span_len[sp]) - t0;
+          n_valid_k = min(min(s_p + n_sink, e_p), p.span_pos[sp] + p.span_len[sp]) - t0;
           key0 = t0 - p.span_pos[sp];
           far = e + 1;
           if (q_lo > q_hi || n_valid_k <= 0) {  // nothing: take the next item into the same slot

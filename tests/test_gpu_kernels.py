@@ -182,6 +182,34 @@ def test_sink_gradients_in_segments(B, S, W, n_sink, lens):
     test_fwd_bwd_matches_oracle("segments", B, S, 4, 2, W, n_sink, lens)
 
 
+@pytest.mark.parametrize("W,n_sink,lens", [(1, 4, [3, 700]), (0, 4, [2, 3, 500, 519]), (2, 6, [5, 4, 4, 500, 5, 511])])
+def test_sink_gradients_of_sequences_shorter_than_n_sink(W, n_sink, lens):
+    """Short sequences whose queries still reach beyond the window: the sink tokens of the next sequence lie within
+    n_sink tokens of their start, and must not end up in their partial sums.  In float32, against the call
+    without segments: both add the same 16-bit terms (below 4 in size: weight 1 x dO) of 2 heads x at most 700
+    queries in float32, in another order: 1400 roundings of a sum that stays below 64, 1400 * 64 * 2^-24 = 5e-3.
+    (A query that sees 6 keys gives each a sixth of its weight, so that against the oracle only the norm stays
+    within the 16-bit bounds of the wider windows.)"""
+    K = _K()
+    S = sum(lens)
+    q, k, v, do = (randn_bf16(1, S, h, D, seed=s) for h, s in ((4, 10), (2, 11), (2, 12), (4, 13)))
+    _, _, _, rdk, rdv = dense_attn_fwd_bwd(q, k, v, do, W, D ** -0.5, n_sink, _cu(lens))
+    q, k, v, do = (x.cuda() for x in (q, k, v, do))
+    cu = torch.tensor(_cu(lens), dtype=torch.int32, device="cuda")
+    out, lse = K.fwd(q, [K.KVSpan(k, v, 0)], W, n_sink, D ** -0.5, 0, cu)
+    plain = K.bwd_workspace(q)
+    assert K.bwd_workspace(q, 2, W, n_sink, len(lens)).numel() > plain.numel()   # this call is cut into segments
+    grads = []
+    for ws in (plain, None):
+        dk, dv = (torch.full(k.shape, float("nan"), dtype=torch.float32, device="cuda") for _ in range(2))
+        K.bwd(q, [K.KVSpan(k, v, 0, dk=dk, dv=dv)], out, lse, do, torch.empty_like(q), W, n_sink, D ** -0.5, 0, cu, workspace=ws)
+        grads.append((dk, dv))
+    K.check_device_status()
+    for name, a, b, ref in zip(("dk", "dv"), grads[1], grads[0], (rdk, rdv)):
+        assert_close(name, a, b, atol=5e-3, rtol=0.0)
+        assert_close(name, a, ref, atol=float("inf"))
+
+
 @pytest.mark.parametrize("cp,S,lens", [(2, 1100, [1098, 1102]), (2, 1152, [2304])])
 def test_sink_gradients_in_segments_over_spans(cp, S, lens):
     """Sink tokens on two spans of a call, and queries that start behind the sink tokens' rank."""
