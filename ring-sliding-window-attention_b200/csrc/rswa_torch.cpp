@@ -16,6 +16,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <cmath>
 #include <cstring>
@@ -170,6 +171,9 @@ class SwaFunction : public torch::autograd::Function<SwaFunction> {
 };
 
 bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu) {
+  // A trace records what goes through the dispatcher: here the allocation of the output, not the kernels that fill
+  // it.  The Python autograd function is recorded as one operator.
+  if (torch::jit::tracer::isTracing()) return false;
   if (!q.is_cuda() || q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
   if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf) return false;
   if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;

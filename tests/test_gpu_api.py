@@ -408,3 +408,16 @@ def test_64_wide_heads(B, S, Hq, Hkv, W, n_sink, lens, dtype, fused):
     ring_swa._kernels.check_device_status()
     for name, a, b in zip(("out", "dq", "dk", "dv"), (out, *grads), (ro, rdq, rdk, rdv)):
         assert_close(name, a, b[0] if lens else b)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_traced_call_computes(grad):
+    """torch.jit.trace records the operators of a call: the attention has to be among them."""
+    import ring_swa
+    a, b = ([randn_bf16(1, 300, h, D, seed=seed + i).cuda().requires_grad_(grad) for i, h in enumerate((4, 2, 2))] for seed in (80, 90))
+
+    def fn(q, k, v):
+        return ring_swa.ring_sliding_window_attn(q, k, v, 100)
+
+    traced = torch.jit.trace(fn, a, check_trace=False)
+    assert torch.equal(traced(*b), fn(*b))
