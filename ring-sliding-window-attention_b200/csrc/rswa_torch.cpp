@@ -174,6 +174,9 @@ bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, con
   // A trace records what goes through the dispatcher: here the allocation of the output, not the kernels that fill
   // it.  The Python autograd function is recorded as one operator.
   if (torch::jit::tracer::isTracing()) return false;
+  // forward-mode derivatives: there are none, and the Python autograd function says so
+  for (const at::Tensor* t : {&q, &k, &v})
+    if (t->_fw_grad(0).defined()) return false;
   if (!q.is_cuda() || q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
   if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf) return false;
   if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;

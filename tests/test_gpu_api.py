@@ -421,3 +421,18 @@ def test_traced_call_computes(grad):
 
     traced = torch.jit.trace(fn, a, check_trace=False)
     assert torch.equal(traced(*b), fn(*b))
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_forward_mode_derivatives_are_refused(head_dim):
+    """There is no forward-mode formula: a tangent on any input is an error, with gradients enabled or not."""
+    import torch.autograd.forward_ad as fwd_ad
+    import ring_swa
+    x = [randn_bf16(1, 300, h, head_dim, seed=80 + i).cuda() for i, h in enumerate((4, 2, 2))]
+    for i in range(3):
+        for grad in (False, True):
+            with fwd_ad.dual_level(), torch.set_grad_enabled(grad):
+                dual = list(x)
+                dual[i] = fwd_ad.make_dual(x[i], torch.ones_like(x[i]))
+                with pytest.raises(NotImplementedError, match="jvp"):
+                    ring_swa.ring_sliding_window_attn(*dual, 100)
