@@ -11,6 +11,8 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -27,7 +29,7 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 constexpr int64_t kHeadDim = 128, kNarrowHeadDim = 64;  // the widths that have kernels
-// per device: the status word the kernels raise and its host mirror (ring_swa/_kernels.py owns both)
+// per device: the status word the kernels raise and its host mirror (made by new_status)
 int32_t* g_status[kMaxDevices] = {nullptr};
 const volatile int32_t* g_mirror[kMaxDevices] = {nullptr};
 
@@ -235,28 +237,40 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// set_status(device index, address of the status word, address of its host mirror)
-PyObject* py_set_status(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 3) {
-    PyErr_SetString(PyExc_TypeError, "set_status takes 3 arguments");
-    return nullptr;
-  }
-  const long dev = PyLong_AsLong(args[0]);
-  void* status = PyLong_AsVoidPtr(args[1]);
-  void* mirror = PyLong_AsVoidPtr(args[2]);
+// new_status(device index) -> (status word, its host mirror): two int32 tensors of one element that live as long as
+// the process.  Not from torch's allocators: the first call on a device may be inside a stream capture, whose
+// allocations belong to the graph (the word would be cleared by every replay) and which allows no pinned ones.
+PyObject* py_new_status(PyObject*, PyObject* arg) {
+  HANDLE_TH_ERRORS
+  const long dev = PyLong_AsLong(arg);
   if (PyErr_Occurred()) return nullptr;
-  if (dev >= 0 && dev < kMaxDevices) {
-    g_status[dev] = static_cast<int32_t*>(status);
-    g_mirror[dev] = static_cast<const volatile int32_t*>(mirror);
+  TORCH_CHECK_VALUE(dev >= 0 && dev < kMaxDevices, "device index ", dev, " is outside the ", kMaxDevices, " this module has status words for");
+  int32_t *word = nullptr, *mirror = nullptr;
+  {
+    const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    C10_CUDA_CHECK(cudaMalloc(&word, sizeof(int32_t)));
+    C10_CUDA_CHECK(cudaHostAlloc(&mirror, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped));
+    *mirror = 0;
+    cudaStream_t stream;  // (of its own: the current one may be capturing)
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    C10_CUDA_CHECK(cudaMemsetAsync(word, 0, sizeof(int32_t), stream));
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    C10_CUDA_CHECK(cudaStreamDestroy(stream));
   }
-  Py_RETURN_NONE;
+  check(rswa_set_status_mirror(word, mirror), "rswa_set_status_mirror");
+  g_status[dev] = word;
+  g_mirror[dev] = mirror;
+  const auto options = at::TensorOptions().dtype(at::kInt);
+  return Py_BuildValue("(NN)", THPVariable_Wrap(at::from_blob(word, {1}, options.device(at::kCUDA, static_cast<c10::DeviceIndex>(dev)))),
+                       THPVariable_Wrap(at::from_blob(mirror, {1}, options)));
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef g_methods[] = {
     {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention)), METH_FASTCALL,
      "attention(q, k, v, window, n_sink, scale, cu_seqlens) -> out or None (the call is not for this path)"},
-    {"set_status", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_set_status)), METH_FASTCALL,
-     "set_status(device_index, status_address, mirror_address)"},
+    {"new_status", py_new_status, METH_O, "new_status(device_index) -> (status word, host mirror)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Single-GPU host path of ring_swa", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

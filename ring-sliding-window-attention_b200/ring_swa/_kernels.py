@@ -5,6 +5,7 @@ All tensors are 4-D here, [batch, tokens, heads, 128]; packed (varlen) callers a
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
@@ -68,6 +69,7 @@ def _dev_key(device: torch.device):
 
 _status = {}    # per device: the word the kernels raise
 _mirrors = {}   # per device: its pinned host copy, written by the kernels themselves
+_status_lock = threading.Lock()
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -79,25 +81,21 @@ def status_word(device: torch.device) -> torch.Tensor:
     key = _dev_key(device)
     word = _status.get(key)
     if word is None:
-        device = torch.device(*key)
-        word = torch.zeros(1, dtype=torch.int32, device=device)
-        if not torch.cuda.is_current_stream_capturing():  # (pinned memory cannot be allocated in a capture)
-            mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
-            _C.check(_C.lib().rswa_set_status_mirror(word.data_ptr(), mirror.data_ptr()), "rswa_set_status_mirror")
-            native_module().set_status(key[1], word.data_ptr(), mirror.data_ptr())
-            _mirrors[key] = mirror
-        _status[key] = word
+        with _status_lock:   # (two threads that make the first call on a device share one word)
+            if key not in _status:
+                word, _mirrors[key] = native_module().new_status(key[1])
+                _status[key] = word
+            word = _status[key]
     return word
 
 
 def _clear_status(device: torch.device) -> None:
     # kernels still queued behind the failed one must have found the word raised before it is cleared, else
-    # they would report once more
+    # they would report once more; and a kernel of the next call, on whichever stream, must find it cleared
     torch.cuda.synchronize(device)
     status_word(device).zero_()
-    mirror = _mirrors.get(_dev_key(device))
-    if mirror is not None:
-        mirror.zero_()
+    torch.cuda.synchronize(device)
+    _mirrors[_dev_key(device)].zero_()
 
 
 def check_device_status(device: Optional[torch.device] = None) -> None:

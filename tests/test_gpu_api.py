@@ -3,6 +3,9 @@ reference's ring functions produced (tests/golden/ref_ring_d128_*.npz), and the 
 behaviour.  Full-size checks use properties that do not need a dense oracle."""
 import glob
 import os
+import subprocess
+import sys
+import threading
 
 import numpy as np
 import pytest
@@ -436,3 +439,61 @@ def test_forward_mode_derivatives_are_refused(head_dim):
                 dual[i] = fwd_ad.make_dual(x[i], torch.ones_like(x[i]))
                 with pytest.raises(NotImplementedError, match="jvp"):
                     ring_swa.ring_sliding_window_attn(*dual, 100)
+
+
+def test_first_call_inside_a_capture():
+    """The first call of a process may be a captured one: its status word must not be the graph's, and a
+    time-out reported later must reach the host.  (A process of its own; the word is raised from the host.)"""
+    code = """
+import torch, ring_swa
+from ring_swa import _kernels as K
+dev = torch.device("cuda")
+q, k, v = (torch.randn(1, 300, h, 128, device=dev, dtype=torch.bfloat16) for h in (4, 2, 2))
+graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+side.wait_stream(torch.cuda.current_stream())
+with torch.cuda.graph(graph, stream=side, capture_error_mode="relaxed"):
+    out = ring_swa.ring_sliding_window_attn(q, k, v, 100)
+graph.replay()
+assert torch.equal(out, ring_swa.ring_sliding_window_attn(q, k, v, 100))
+from ring_swa import _native
+assert _native.attention(q, k, v, 100, 0, None, None) is not None   # later calls take the C++ path
+K.status_word(dev).fill_(103)
+out.zero_()
+graph.replay()                                  # the word stays raised: no work, and the host hears of it
+torch.cuda.synchronize()
+assert not out.any()
+try:
+    ring_swa.ring_sliding_window_attn(q, k, v, 100)
+    raise SystemExit("not reported")
+except RuntimeError as e:
+    assert "bounded device-side wait" in str(e), e
+graph.replay()
+assert torch.equal(out, ring_swa.ring_sliding_window_attn(q, k, v, 100))
+"""
+    import ring_swa
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(ring_swa.__file__)))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_first_calls_of_threads_share_one_status_word():
+    import ring_swa
+    from ring_swa import _kernels as K
+    dev = torch.device("cuda")
+    K.check_device_status()
+    K._status.pop(K._dev_key(dev)), K._mirrors.pop(K._dev_key(dev))   # as in a process that has made no call yet
+    words = []
+    threads = [threading.Thread(target=lambda: words.append(K.status_word(dev))) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(words) == 8 and all(w is words[0] for w in words)
+    words[0].fill_(103)
+    q = torch.zeros(1, 256, 2, D, dtype=torch.bfloat16, device=dev)
+    ring_swa.ring_sliding_window_attn(q, q, q, 10)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="bounded device-side wait"):
+        ring_swa.ring_sliding_window_attn(q, q, q, 10)
+    ring_swa.ring_sliding_window_attn(q, q, q, 10)
+    K.check_device_status()
