@@ -95,6 +95,48 @@ void check(int rc, const char* what) {
   TORCH_CHECK(false, what, ": ", rswa_last_error(), " (code ", rc, ")");
 }
 
+// q, k, v (and cu_seqlens) are what the kernels take and fit together.
+bool fits(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu) {
+  if (!q.is_cuda() || q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
+  if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf) return false;
+  if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;
+  if (k.device() != q.device() || v.device() != q.device()) return false;
+  if (q.dim() != (cu.defined() ? 3 : 4) || k.dim() != q.dim() || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return false;
+  if ((q.size(-1) != kHeadDim && q.size(-1) != kNarrowHeadDim) || k.size(-1) != q.size(-1)) return false;
+  const Dims dq = dims_of(q), dk = dims_of(k);
+  if (dq.batch != dk.batch || dq.tokens != dk.tokens || dq.heads % dk.heads != 0) return false;
+  if (dq.batch > 0x7fffffff || dq.tokens > 0x7fffffff || dq.heads > 0x7fffffff) return false;
+  if (cu.defined() && (cu.device() != q.device() || cu.scalar_type() != at::kInt || cu.dim() != 1 || !cu.is_contiguous() || cu.numel() < 2))
+    return false;
+  return true;
+}
+
+bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu) {
+  // A trace records what goes through the dispatcher: here the allocation of the output, not the kernels that fill
+  // it.  The Python autograd function is recorded as one operator.
+  if (torch::jit::tracer::isTracing()) return false;
+  // forward-mode derivatives: there are none, and the Python autograd function says so
+  for (const at::Tensor* t : {&q, &k, &v})
+    if (t->_fw_grad(0).defined()) return false;
+  if (!fits(q, k, v, cu)) return false;
+  const int dev = q.get_device();
+  if (dev < 0 || dev >= kMaxDevices || g_mirror[dev] == nullptr || *g_mirror[dev] != 0) return false;
+  return dev == c10::cuda::current_device();
+}
+
+// Tensors that a saved-tensor hook hands back to the backward may be anything (another device, type, shape or
+// layout than was saved): only those that the kernels can address are let through.
+bool saved_as_expected(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out, const at::Tensor& lse,
+                       const at::Tensor& cu, const at::Tensor& dout) {
+  if (!fits(q, k, v, cu) || q.sizes() != dout.sizes() || q.device() != dout.device() || q.scalar_type() != dout.scalar_type()) return false;
+  if (out.sizes() != q.sizes() || out.scalar_type() != q.scalar_type() || out.device() != q.device()) return false;
+  for (const at::Tensor* t : {&q, &k, &v, &out})
+    if (t->stride(-1) != 1) return false;
+  const Dims d = dims_of(q);
+  return k.strides() == v.strides() && lse.sizes() == at::IntArrayRef({d.batch, d.heads, d.tokens}) && lse.scalar_type() == at::kFloat &&
+         lse.device() == q.device() && lse.is_contiguous();
+}
+
 at::Tensor forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu, const Call& c, at::Tensor& lse) {
   const Dims d = dims_of(q);
   at::Tensor out = at::empty_like(q);
@@ -133,6 +175,8 @@ class SwaFunction : public torch::autograd::Function<SwaFunction> {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4], &cu = saved[5];
     const Call c = {ctx->saved_data["window"].toInt(), ctx->saved_data["n_sink"].toInt(), ctx->saved_data["scale"].toDouble()};
+    TORCH_CHECK_VALUE(saved_as_expected(q, k, v, out, lse, cu, grads[0]),
+                      "rswa_bwd: a saved tensor came back from a hook on another device or with another type, shape or layout");
     const c10::cuda::CUDAGuard guard(q.device());
     const at::Tensor dout = dense(grads[0]);
     at::Tensor dq = at::empty_like(q);
@@ -171,30 +215,6 @@ class SwaFunction : public torch::autograd::Function<SwaFunction> {
     return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
-
-bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu) {
-  // A trace records what goes through the dispatcher: here the allocation of the output, not the kernels that fill
-  // it.  The Python autograd function is recorded as one operator.
-  if (torch::jit::tracer::isTracing()) return false;
-  // forward-mode derivatives: there are none, and the Python autograd function says so
-  for (const at::Tensor* t : {&q, &k, &v})
-    if (t->_fw_grad(0).defined()) return false;
-  if (!q.is_cuda() || q.layout() != at::kStrided || k.layout() != at::kStrided || v.layout() != at::kStrided) return false;
-  if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf) return false;
-  if (k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;
-  if (k.device() != q.device() || v.device() != q.device()) return false;
-  const int dev = q.get_device();
-  if (dev < 0 || dev >= kMaxDevices || g_mirror[dev] == nullptr || *g_mirror[dev] != 0) return false;
-  if (dev != c10::cuda::current_device()) return false;
-  if (q.dim() != (cu.defined() ? 3 : 4) || k.dim() != q.dim() || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return false;
-  if ((q.size(-1) != kHeadDim && q.size(-1) != kNarrowHeadDim) || k.size(-1) != q.size(-1)) return false;
-  const Dims dq = dims_of(q), dk = dims_of(k);
-  if (dq.batch != dk.batch || dq.tokens != dk.tokens || dq.heads % dk.heads != 0) return false;
-  if (dq.batch > 0x7fffffff || dq.tokens > 0x7fffffff || dq.heads > 0x7fffffff) return false;
-  if (cu.defined() && (!cu.is_cuda() || cu.get_device() != dev || cu.scalar_type() != at::kInt || cu.dim() != 1 || !cu.is_contiguous() || cu.numel() < 2))
-    return false;
-  return true;
-}
 
 // attention(q, k, v, window, n_sink, scale or None, cu_seqlens or None) -> out, or None (see above)
 PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {

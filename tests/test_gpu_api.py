@@ -497,3 +497,57 @@ def test_first_calls_of_threads_share_one_status_word():
         ring_swa.ring_sliding_window_attn(q, q, q, 10)
     ring_swa.ring_sliding_window_attn(q, q, q, 10)
     K.check_device_status()
+
+
+def _grads(fn, x, do):
+    x = [t.detach().requires_grad_(True) for t in x]
+    out = fn(*x)
+    return (out.detach(), *torch.autograd.grad(out, x, do))
+
+
+@pytest.mark.parametrize("varlen", [False, True])
+def test_saved_tensor_hooks_and_checkpointing(varlen):
+    """What the backward needs goes through saved-tensor hooks: offloading and both forms of activation
+    checkpointing give the same bits."""
+    import ring_swa
+    from torch.utils.checkpoint import checkpoint
+    x = [randn_bf16(1, 400, h, D, seed=30 + i).cuda() for i, h in enumerate((4, 2, 2))]
+    do = randn_bf16(1, 400, 4, D, seed=33).cuda()
+    if varlen:
+        x, do = [t[0] for t in x], do[0]
+        cu = torch.tensor([0, 130, 400], dtype=torch.int32, device="cuda")
+
+        def fn(q, k, v):
+            return ring_swa.ring_streaming_llm_attn_varlen(q, k, v, 100, cu, cp_size=1)
+    else:
+        def fn(q, k, v):
+            return ring_swa.ring_sliding_window_attn(q, k, v, 100)
+    ref = _grads(fn, x, do)
+    with torch.autograd.graph.save_on_cpu(pin_memory=True):
+        got = _grads(fn, x, do)
+    assert all(torch.equal(a, b) for a, b in zip(got, ref))
+    assert all(torch.equal(a, b) for a, b in zip(_grads(lambda *t: checkpoint(fn, *t, use_reentrant=False), x, do), ref))
+    leaves = [t.detach().requires_grad_(True) for t in x]
+    checkpoint(fn, *leaves, use_reentrant=True).backward(do)
+    assert all(torch.equal(t.grad, b) for t, b in zip(leaves, ref[1:]))
+
+
+@pytest.mark.parametrize("what", ["device", "dtype", "shape", "layout"])
+@pytest.mark.parametrize("which", range(5))
+def test_saved_tensors_that_come_back_different_are_refused(which, what):
+    """A hook may hand anything back to the backward; what the kernels cannot address is an error before any launch."""
+    import ring_swa
+    x = [randn_bf16(1, 256, h, D, seed=30 + i).cuda() for i, h in enumerate((4, 2, 2))]
+    do = randn_bf16(1, 256, 4, D, seed=33).cuda()
+    change = {"device": lambda t: t.cpu(), "dtype": lambda t: t.double(), "shape": lambda t: t[..., :-8].contiguous(),
+              "layout": lambda t: t.transpose(-1, -2).contiguous().transpose(-1, -2)}[what]
+    n = [0]
+
+    def unpack(t):   # called once for each of q, k, v, out, lse
+        n[0] += 1
+        return change(t) if n[0] - 1 == which else t
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), unpack):
+        with pytest.raises((ValueError, RuntimeError)):
+            _grads(lambda *t: ring_swa.ring_sliding_window_attn(*t, 100), x, do)
+    assert n[0] == 5
