@@ -58,7 +58,17 @@ bool dense_enough(const at::Tensor& t) {
     if (st[i] <= 0 || st[i] % 8 != 0) return false;
   return true;
 }
-at::Tensor dense(const at::Tensor& t) { return dense_enough(t) ? t : t.contiguous(); }
+at::Tensor dense(const at::Tensor& t) {
+  if (dense_enough(t)) return t;
+  const at::Tensor c = t.contiguous();
+  // contiguous() returns a tensor that is contiguous already as it is, unaligned or with odd strides of its
+  // dimensions of size 1.  The library refuses those at 128 elements per head; at 64 they are copied, as by the
+  // zero padding that other widths go through.
+  const bool batch_of_one = t.dim() == 4 && t.size(0) == 1 && t.stride(0) == 0;  // (the library knows what to do)
+  if (t.size(-1) == kNarrowHeadDim && c.data_ptr() == t.data_ptr() && !dense_enough(batch_of_one ? c.select(0, 0) : c))
+    return t.clone(at::MemoryFormat::Contiguous);
+  return c;
+}
 
 struct Call {
   int64_t window, n_sink;
@@ -245,6 +255,10 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (k.strides() != v.strides()) {
       k = k.contiguous();
       v = v.contiguous();
+      if (k.strides() != v.strides()) {  // (in dimensions of size 1)
+        k = k.clone(at::MemoryFormat::Contiguous);
+        v = v.clone(at::MemoryFormat::Contiguous);
+      }
     }
     if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
       out = SwaFunction::apply(q, k, v, cu.defined() ? std::optional<at::Tensor>(cu) : std::nullopt, window, n_sink, scale);

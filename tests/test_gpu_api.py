@@ -551,3 +551,41 @@ def test_saved_tensors_that_come_back_different_are_refused(which, what):
         with pytest.raises((ValueError, RuntimeError)):
             _grads(lambda *t: ring_swa.ring_sliding_window_attn(*t, 100), x, do)
     assert n[0] == 5
+
+
+def _odd(t, how):
+    """t's values in a tensor that is contiguous and yet not what a TMA descriptor can address."""
+    if how == "unaligned":
+        return torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)[1:1 + t.numel()].view(t.shape).copy_(t)
+    assert t.shape[0] == 1
+    return t.as_strided(t.shape, ({"batch stride 3": 3, "batch stride 0": 0}[how],) + t.stride()[1:])
+
+
+@pytest.mark.parametrize("how", ["unaligned", "batch stride 3", "batch stride 0"])
+@pytest.mark.parametrize("which", range(4))
+def test_64_wide_heads_of_any_alignment(which, how):
+    """Heads of 64 elements: q, k, v and the gradient of the output at any address and with any stride of a batch
+    of one, as when they were padded into tensors of their own."""
+    import ring_swa
+    x = [randn_bf16(1, 300, h, 64, seed=40 + i).cuda() for i, h in enumerate((4, 2, 2, 4))]
+
+    def fn(q, k, v):
+        return ring_swa.ring_sliding_window_attn(q, k, v, 100)
+
+    ref = _grads(fn, x[:3], x[3])
+    x[which] = _odd(x[which], how)
+    assert x[which].is_contiguous()
+    assert all(torch.equal(a, b) for a, b in zip(_grads(fn, x[:3], x[3]), ref))
+
+
+def test_keys_and_values_with_different_strides_of_a_batch_of_one():
+    import ring_swa
+    for d in (64, D):
+        x = [randn_bf16(1, 300, h, d, seed=40 + i).cuda() for i, h in enumerate((4, 2, 2, 4))]
+
+        def fn(q, k, v):
+            return ring_swa.ring_sliding_window_attn(q, k, v, 100)
+
+        ref = _grads(fn, x[:3], x[3])
+        x[1] = _odd(x[1], "batch stride 0")
+        assert all(torch.equal(a, b) for a, b in zip(_grads(fn, x[:3], x[3]), ref))
