@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -125,6 +126,8 @@ bool ordinary(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, con
   // A trace records what goes through the dispatcher: here the allocation of the output, not the kernels that fill
   // it.  The Python autograd function is recorded as one operator.
   if (torch::jit::tracer::isTracing()) return false;
+  // vmap, torch.func.grad and the like: the Python autograd function says that it does not support them
+  if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode)) return false;
   // forward-mode derivatives: there are none, and the Python autograd function says so
   for (const at::Tensor* t : {&q, &k, &v})
     if (t->_fw_grad(0).defined()) return false;
@@ -233,8 +236,8 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "attention takes 7 arguments");
     return nullptr;
   }
-  for (int i = 0; i < 3; ++i)
-    if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
+  for (int i = 0; i < 3; ++i)  // (Tensor or Parameter: the result of another subclass is of that type)
+    if (!THPVariable_CheckTypeExact(Py_TYPE(args[i]))) Py_RETURN_NONE;
   if (args[6] != Py_None && !THPVariable_Check(args[6])) Py_RETURN_NONE;
   const int64_t window = PyLong_AsLongLong(args[3]), n_sink = PyLong_AsLongLong(args[4]);
   double scale = args[5] == Py_None ? 0. : PyFloat_AsDouble(args[5]);

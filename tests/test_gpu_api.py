@@ -589,3 +589,26 @@ def test_keys_and_values_with_different_strides_of_a_batch_of_one():
         ref = _grads(fn, x[:3], x[3])
         x[1] = _odd(x[1], "batch stride 0")
         assert all(torch.equal(a, b) for a, b in zip(_grads(fn, x[:3], x[3]), ref))
+
+
+def test_subclasses_and_function_transforms():
+    """A subclass's result is of its type, and transforms of torch.func are refused by the autograd function."""
+    import ring_swa
+
+    class Sub(torch.Tensor):
+        pass
+
+    x = [randn_bf16(1, 300, h, D, seed=50 + i).cuda() for i, h in enumerate((4, 2, 2))]
+
+    def fn(q, k, v):
+        return ring_swa.ring_sliding_window_attn(q, k, v, 100)
+
+    out = fn(*x)
+    for i in range(3):
+        got = fn(*[t.as_subclass(Sub) if j == i else t for j, t in enumerate(x)])
+        assert type(got) is (Sub if i == 0 else torch.Tensor) and torch.equal(got, out)
+    assert type(fn(*[torch.nn.Parameter(t) for t in x])) is torch.Tensor
+    for call in (lambda: torch.func.vmap(fn)(*[t[None] for t in x]), lambda: torch.func.vmap(fn, in_dims=(0, None, None))(x[0][None], *x[1:]),
+                 lambda: torch.func.grad(lambda q: fn(q, *x[1:]).float().sum())(x[0])):
+        with pytest.raises(RuntimeError, match="setup_context"):
+            call()
