@@ -637,8 +637,14 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
 // A handful of 512-byte rows per block: latency, 4 us where it replaced a serial chain of milliseconds.
 template <bool kBf16>
 __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ BwdKernelParams p) {
-  const int r = blockIdx.x % p.n_sink, i = blockIdx.x / p.n_sink;
-  const int hk = blockIdx.y, b = blockIdx.z;
+  // (one grid dimension: the others end at 65535, and a batch need not)
+  const int n_seq = p.cu == nullptr ? 1 : p.n_seqs + 1;
+  int idx = blockIdx.x;
+  const int r = idx % p.n_sink;
+  idx /= p.n_sink;
+  const int i = idx % n_seq;
+  idx /= n_seq;
+  const int hk = idx % p.hkv, b = idx / p.hkv;
   int s, e, q_lo, q_hi;
   far_range(p, i, 0, s, e, q_lo, q_hi);
   const int t = s + r;
@@ -712,7 +718,7 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool e
 int launch_sink_sum(const BwdKernelParams& kp, int dtype, cudaStream_t stream) {
   if (kp.far_segs > 0) {
     const int n_seq = kp.cu == nullptr ? 1 : kp.n_seqs + 1;
-    const dim3 grid(static_cast<unsigned>(n_seq * kp.n_sink), static_cast<unsigned>(kp.hkv), static_cast<unsigned>(kp.batch));
+    const unsigned grid = static_cast<unsigned>(n_seq * kp.n_sink) * kp.hkv * kp.batch;
     if (dtype == RSWA_DTYPE_BF16) sink_sum_kernel<true><<<grid, 2 * kp.head_dim, 0, stream>>>(kp);
     else sink_sum_kernel<false><<<grid, 2 * kp.head_dim, 0, stream>>>(kp);
     count_launches(1);

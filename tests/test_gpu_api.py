@@ -612,3 +612,12 @@ def test_subclasses_and_function_transforms():
                  lambda: torch.func.grad(lambda q: fn(q, *x[1:]).float().sum())(x[0])):
         with pytest.raises(RuntimeError, match="setup_context"):
             call()
+
+
+def test_sink_gradients_of_more_than_65535_rows():
+    """Blocks of the sink sums are one per row and more: a batch beyond the limit of a grid's y and z dimensions.  (385
+    tokens: the shortest axis whose sink gradients are summed from segments.)  Equal rows give equal bits."""
+    import ring_swa
+    x = [torch.randn(8, 385, 1, 64, device="cuda").bfloat16().repeat(8192, 1, 1, 1) for _ in range(4)]
+    for t in _grads(lambda q, k, v: ring_swa.ring_streaming_llm_attn(q, k, v, 60), x[:3], x[3]):
+        assert torch.equal(t[:8], t[-8:])
