@@ -12,7 +12,9 @@ namespace rswa {
 int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream);
 int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool early, cudaStream_t stream);
 int launch_sink_sum(const BwdKernelParams& kp, int dtype, cudaStream_t stream);
-int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, int* counters, cudaStream_t stream);
+int launch_begin_call(const BwdKernelParams& next, int* counters, cudaStream_t stream);
+int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, const BwdKernelParams& next, int* counters,
+                 cudaStream_t stream);
 int launch_dq(const BwdKernelParams& kp, int dtype, bool early, cudaStream_t stream);
 
 static thread_local char g_err[512] = "";
@@ -237,10 +239,10 @@ int sm_count() {
 // sink token) and packs of sequences shorter than a tile on average (their segments would be mostly empty).
 struct FarPlan {
   int segs, chunk, slots;
-  int64_t bytes;
+  int64_t sum_bytes, bytes;  // partial sums; with the list of segments behind them
 };
 static FarPlan far_plan(int batch, int q_len, int hkv, int window, int n_sink, int n_seqs) {
-  FarPlan f = {0, 0, 0, 0};
+  FarPlan f = {0, 0, 0, 0, 0};
   const int n_tiles = (q_len + kTile - 1) / kTile;
   const int per_key = window / kTile + 2;
   if (n_sink <= 0 || n_sink > 16 || n_tiles / 2 < per_key || n_seqs > n_tiles) return f;
@@ -248,7 +250,8 @@ static FarPlan far_plan(int batch, int q_len, int hkv, int window, int n_sink, i
   f.chunk = chunk_tiles * kTile;
   f.segs = (n_tiles + chunk_tiles - 1) / chunk_tiles + n_seqs;
   f.slots = f.segs + (n_seqs > 0 ? n_seqs + 1 : 1);
-  f.bytes = static_cast<int64_t>(batch) * hkv * f.slots * n_sink * 2 * kHeadDim * sizeof(float);
+  f.sum_bytes = static_cast<int64_t>(batch) * hkv * f.slots * n_sink * 2 * kHeadDim * sizeof(float);
+  f.bytes = f.sum_bytes + (f.segs + 1) * static_cast<int64_t>(sizeof(int));
   return f;
 }
 
@@ -387,13 +390,6 @@ static int bwd_call(const rswa_bwd_params_t* p, int head_dim, void* stream_) {
   float* delta = static_cast<float*>(p->workspace);
   float* lse2 = delta + static_cast<int64_t>(g.batch) * g.n_q_heads * q_len_pad;
   int* dq_counter = reinterpret_cast<int*>(lse2 + static_cast<int64_t>(g.batch) * g.n_q_heads * q_len_pad);
-  if (!(p->flags & RSWA_BWD_INIT)) {  // both work counters; with INIT the delta kernel resets them
-    cudaError_t e = cudaMemsetAsync(dq_counter, 0, 2 * sizeof(int), static_cast<cudaStream_t>(stream_));
-    if (e != cudaSuccess) {
-      set_error("rswa_bwd: cudaMemsetAsync: %s", cudaGetErrorString(e));
-      return RSWA_E_CUDA;
-    }
-  }
 
   // kq: every span (the dQ kernel sums over all keys); kk: only the spans whose dK/dV are wanted
   BwdKernelParams kq, kk;
@@ -462,17 +458,20 @@ static int bwd_call(const rswa_bwd_params_t* p, int head_dim, void* stream_) {
   kk.span_tile0[n_k] = total_tiles;
   kk.n_spans = n_k;
   const FarPlan far = far_plan(g.batch, g.q_len, g.n_kv_heads, g.window, g.n_sink, g.cu_seqlens ? g.n_seqs : 0);
-  if (far.bytes > 0 && n_k > 0 && p->workspace_bytes >= need + far.bytes) {
+  // (without packed sequences the kernels' own rule, far_split, is known here)
+  const int far_queries = g.q_len - (g.window + 1 > g.q_pos_start ? g.window + 1 - g.q_pos_start : 0);
+  const bool far_any = g.cu_seqlens != nullptr || far_queries > far.chunk;
+  if (far.bytes > 0 && far_any && n_k > 0 && p->workspace_bytes >= need + far.bytes) {
     kk.far_segs = far.segs;
     kk.far_chunk = far.chunk;
     kk.far_slots = far.slots;
     kk.far_ws = reinterpret_cast<float*>(static_cast<uint8_t*>(p->workspace) + need);
+    kk.far_list = reinterpret_cast<int*>(static_cast<uint8_t*>(p->workspace) + need + far.sum_bytes);
   }
 
-  if (p->flags & RSWA_BWD_INIT) {
-    rc = launch_delta(*p, delta, lse2, q_len_pad, dq_counter, stream);
-    if (rc) return rc;
-  }
+  // (both kernels also reset the work counters and list the segments)
+  rc = (p->flags & RSWA_BWD_INIT) ? launch_delta(*p, delta, lse2, q_len_pad, kk, dq_counter, stream) : launch_begin_call(kk, dq_counter, stream);
+  if (rc) return rc;
   // The two tensor kernels overlap: the dQ kernel takes over the SMs that the dK/dV kernel runs out of work for
   // (20 of 148 have none from the start, at 4096 tokens of 32/4 heads).  Not where an event between the two is asked
   // for, nor where dq is written over an input that the dK/dV kernel may still read.

@@ -87,7 +87,7 @@ static_assert(kBwdSmemBytes <= 232448, "shared memory budget");
 // kD: width of a head, 128 or 64.
 template <int kD, bool kBf16, bool kPlain>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
+rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_tile_items) {
   constexpr uint32_t kLoadBytes = kD / 64 * kBoxBytes;  // what a tile holds (its slots in shared memory are kTileBytes apart)
   constexpr uint32_t kStageTxBytes = kLoadBytes + kRowBytes;
   const int* const cu_seq = kPlain ? nullptr : p.cu;
@@ -146,7 +146,6 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
   const uint32_t tmem = ctl->tmem_base;
   const uint32_t tDK = tmem, tDV = tmem + 128, tS = tmem + 256, tB = tmem + 384;
   volatile int* err = &ctl->err;
-  const int n_work = (ctl->err != 0) ? 0 : n_items;
   constexpr uint32_t kTile16 = kTileBytes >> 4;
 
   if (warp < 4) {
@@ -155,6 +154,9 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
       // ------------------------------------------------------------------ item geometry + TMA producer
       int gi = 0;  // query tiles loaded so far, all items (ring stages and barrier phases)
       int nk = 0;  // items with work so far
+      // far items (see BwdKernelParams) come first: they are the longest where the segments' sequences are long
+      const int n_far = !kPlain && p.far_segs > 0 ? p.far_list[0] * n_spans : 0;  // per KV head and batch row
+      const int n_work = (ctl->err != 0) ? 0 : n_tile_items + n_far * p.hkv * p.batch;
       for (int n = 0;; ++n) {
         const int slot = n & 1;
         // (waiting for the same phase again, after an item that turned out to be empty, returns at once)
@@ -175,12 +177,12 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         const int hk = idx % p.hkv;
         idx /= p.hkv;
         int sp = 0, key0, n_valid_k, t0, q_lo, q_hi, far = 0;
-        if (!kPlain && idx < p.far_segs * n_spans) {
+        if (!kPlain && idx < n_far) {
           // The queries of one segment beyond the window of the sink tokens of their sequence: a tile that
           // starts at the first of those this span holds (a TMA load may start at any token).  Its rows end
           // with the sink tokens and with the sequence: in a sequence shorter than n_sink the next rows are sink
           // tokens of the NEXT one, whose partial sums would go to the slots of this one's.
-          const int e = idx / n_spans;
+          const int e = p.far_list[1 + idx / n_spans];
           sp = idx % n_spans;
           const int i = far_sequence(p, e);
           int s_p, e_p;
@@ -189,12 +191,12 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
           n_valid_k = min(min(s_p + n_sink, e_p), p.span_pos[sp] + p.span_len[sp]) - t0;
           key0 = t0 - p.span_pos[sp];
           far = e + 1;
-          if (q_lo > q_hi || n_valid_k <= 0) {  // nothing: take the next item into the same slot
+          if (n_valid_k <= 0) {  // none of them on this span: take the next item into the same slot
             --n;
             continue;
           }
         } else {
-          const int kt_g = kPlain ? idx : idx - p.far_segs * n_spans;
+          const int kt_g = idx - n_far;
           while (sp + 1 < n_spans && kt_g >= p.span_tile0[sp + 1]) ++sp;
           key0 = (kt_g - p.span_tile0[sp]) * kTile;  // token offset inside the span
           n_valid_k = min(kTile, p.span_len[sp] - key0);
@@ -204,7 +206,7 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
           int s_last, e_last;
           seq_of(cu_seq, n_seqs, t_last, s_last, e_last);
           int pmax;
-          if (n_sink > 0 && p.far_segs == 0 && s_last + n_sink > t0) {
+          if (n_sink > 0 && s_last + n_sink > t0 && !far_split(p, s_last, e_last)) {
             pmax = e_last - 1;  // the tile holds a sink token: every later query of that sequence
           } else {
             pmax = (e_last - 1 - t_last > p.window) ? t_last + p.window : e_last - 1;
@@ -448,10 +450,10 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_items) {
         int s_t, e_t;
         const int i_t = seq_of(cu_seq, n_seqs, t, s_t, e_t);
         const bool is_sink = t < s_t + n_sink;
-        const bool split = !kPlain && p.far_segs > 0;
+        const bool split = !kPlain && is_sink && far_split(p, s_t, e_t);
         p_hi = ((is_sink && !split) || e_t - 1 - t <= p.window) ? e_t - 1 : t + p.window;
         p_hi = min(p_hi, q_end_pos - 1);
-        if (split && is_sink && min(e_t, q_end_pos) - 1 - t > p.window) {
+        if (split && min(e_t, q_end_pos) - 1 - t > p.window) {
           const int slot_ws = gm.far ? gm.far - 1 : p.far_segs + i_t;
           ws = p.far_ws + ((static_cast<long long>(gm.b * p.hkv + gm.hk) * p.far_slots + slot_ws) * n_sink + (t - s_t)) * 256 + half * (kD / 2);
         }
@@ -648,7 +650,8 @@ __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ B
   int s, e, q_lo, q_hi;
   far_range(p, i, 0, s, e, q_lo, q_hi);
   const int t = s + r;
-  if (t >= e || min(e, p.q_pos_start + p.q_len) - 1 - t <= p.window) return;  // no far query: dk / dv hold the result
+  // no segments, or no far query of this token: dk / dv hold the result
+  if (t >= e || !far_split(p, s, e) || min(e, p.q_pos_start + p.q_len) - 1 - t <= p.window) return;
   int sp = 0;
   while (sp < p.n_spans && (t < p.span_pos[sp] || t >= p.span_pos[sp] + p.span_len[sp])) ++sp;
   if (sp == p.n_spans) return;
@@ -676,9 +679,9 @@ __global__ void __launch_bounds__(256) sink_sum_kernel(const __grid_constant__ B
 }  // namespace
 
 int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool early, cudaStream_t stream) {
-  // far items (see BwdKernelParams) come first: they are the longest where the segments' sequences are long
-  const long long n_cta = (static_cast<long long>(total_key_tiles) + static_cast<long long>(kp.far_segs) * kp.n_spans) * kp.hkv * kp.batch;
-  if (n_cta <= 0) return RSWA_OK;
+  const long long n_tile_items = static_cast<long long>(total_key_tiles) * kp.hkv * kp.batch;
+  const long long n_cta = n_tile_items + static_cast<long long>(kp.far_segs) * kp.n_spans * kp.hkv * kp.batch;  // (at most)
+  if (n_tile_items <= 0) return RSWA_OK;
   if (n_cta > 0x7fffffffLL) {
     set_error("rswa_bwd: too many key tiles (%lld)", n_cta);
     return RSWA_E_ARG;
@@ -705,7 +708,7 @@ int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool e
   }
   // one CTA per SM (shared memory and TMEM allow no more), each striding over the items
   const long long n_grid = n_cta < sm_count() ? n_cta : sm_count();
-  e = launch_kernel(kern, dim3(static_cast<unsigned>(n_grid)), kBwdThreads, kBwdSmemBytes, stream, early, kp, static_cast<int>(n_cta));
+  e = launch_kernel(kern, dim3(static_cast<unsigned>(n_grid)), kBwdThreads, kBwdSmemBytes, stream, early, kp, static_cast<int>(n_tile_items));
   count_launches(1);
   if (e != cudaSuccess) {
     set_error("rswa_bwd: launch: %s", cudaGetErrorString(e));

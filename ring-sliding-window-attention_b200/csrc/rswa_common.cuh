@@ -83,11 +83,12 @@ struct BwdKernelParams {
   int* mirror;  // host-visible copy of the status word (or null)
   // Sink tokens are seen by every later query of their sequence.  When far_segs > 0 the dK/dV kernel treats
   // the queries beyond a sink token's window separately: the query axis is cut into far_segs segments
-  // (see far_segment), each a work item of its own per KV head, whose dK / dV of the sink rows go to far_ws
-  // as partial sums ([batch, hkv, far_segs + sequences, n_sink, 2, 128] fp32; the rows' windowed part goes to
-  // the slot far_segs + sequence) and are added up by sink_sum_kernel.
+  // (see far_range); those that hold such queries (far_split) are work items of their own per KV head, whose dK / dV of
+  // the sink rows go to far_ws as partial sums ([batch, hkv, far_segs + sequences, n_sink, 2, 128] fp32; the rows'
+  // windowed part goes to the slot far_segs + sequence) and are added up by sink_sum_kernel.
   int far_segs, far_chunk, far_slots;  // far_chunk: positions per chunk, a multiple of the tile
   float* far_ws;
+  int* far_list;  // number of segments that are work items, then these segments (written by begin_call)
 };
 
 // Programmatic dependent launch.  The tensor kernels are launched with the attribute that lets a kernel start while
@@ -150,6 +151,15 @@ __device__ __forceinline__ void far_range(const BwdKernelParams& p, int i, int j
   const int z = j + 1 < n_chunks ? a + p.far_chunk : q_end;
   q_lo = max(max(s, a), s > 0x7ffffffe - p.window ? 0x7fffffff : s + p.window + 1);
   q_hi = min(e, z) - 1;
+}
+// Whether the sequence [s, e) is treated that way: only if the queries beyond the window of its first token are more
+// than one segment.  Fewer cost the sink tokens' key tile at most as many tile products again as an ordinary one has,
+// and a segment item (its loads, its partial sums) costs more: 32768 tokens in 250 sequences of 131, 32/8
+// heads, window 64, 4 sink tokens: 1086 us a training step without segments, 1280 us with one for each sequence.
+__device__ __forceinline__ bool far_split(const BwdKernelParams& p, int s, int e) {
+  if (p.far_segs == 0) return false;
+  const int first = s > 0x7ffffffe - p.window ? 0x7fffffff : s + p.window + 1;
+  return min(e, p.q_pos_start + p.q_len) - max(first, p.q_pos_start) > p.far_chunk;
 }
 // number of sequence starts among the first e of the merged boundaries (starts first on ties)
 __device__ __forceinline__ int far_sequence(const BwdKernelParams& p, int e) {

@@ -167,9 +167,13 @@ def test_spans_emulated_ranks(cp, S, W, n_sink, lens):
 
 
 # The queries beyond a sink token's window are cut into segments of 4 query tiles (window below 256 tokens) at
-# sequence starts, where the axis has at least twice as many tiles as a key's window.
+# sequence starts, where the axis has at least twice as many tiles as a key's window and a sequence more such
+# queries than a segment holds.
 @pytest.mark.parametrize("B,S,W,n_sink,lens", [
-    (1, 512, 60, 1, None),                        # one segment: the smallest axis that is cut
+    (1, 512, 60, 1, None),                        # no more than one segment: not cut
+    (1, 573, 60, 1, None),
+    (1, 574, 60, 1, None),                        # ... one more query: the smallest axis that is cut
+    (1, 1800, 60, 3, [573, 574, 80, 573]),        # the same of sequences
     (2, 1030, 60, 2, None),                       # three segments, the last of six tokens
     (1, 1400, 300, 16, None),                     # the most sink tokens that are kept as partial sums
     (1, 1400, 100, 17, None),                     # ... one more: not cut
