@@ -347,7 +347,7 @@ extern "C" int64_t rswa_bwd_workspace_bytes(int32_t batch, int32_t q_len, int32_
   if (batch <= 0 || q_len <= 0 || n_q_heads <= 0 || head_dim != kHeadDim) return -1;
   const int64_t q_len_pad = (static_cast<int64_t>(q_len) + kTile - 1) / kTile * kTile;
   // two fp32 rows per (batch, head): delta = rowsum(dO * O) and lse * log2(e), padded to whole tiles;
-  // then 256 bytes that hold the work counters of the dQ and dK/dV kernels
+  // then 256 bytes that hold the work counters of the dQ and dK/dV kernels and the gate between them
   return 2 * static_cast<int64_t>(batch) * n_q_heads * q_len_pad * 4 + 256;
 }
 
@@ -477,6 +477,7 @@ static int bwd_call(const rswa_bwd_params_t* p, int head_dim, void* stream_) {
   // for, nor where dq is written over an input that the dK/dV kernel may still read.
   const bool overlap = (p->flags & RSWA_BWD_INIT) && total_tiles > 0 && want_dq && !p->ev_main_start && !p->ev_main_mid &&
                        p->dq != p->q && p->dq != p->dout;
+  kk.gate = kq.gate = overlap ? dq_counter + 2 : nullptr;
   if (p->ev_main_start) cudaEventRecord(static_cast<cudaEvent_t>(p->ev_main_start), stream);
   if (total_tiles > 0) {
     kk.dkv_counter = dq_counter + 1;

@@ -36,7 +36,7 @@ __device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
 // 1.5 us each: 65536 tokens in 400 sequences, 32/8 heads, window 1000 (no sequence reaches beyond it): 2114 us a training
 // step, 2084 with the list, 2077 without anything for sink tokens.
 __device__ __forceinline__ void begin_call(const BwdKernelParams& p, int* counters) {
-  if (threadIdx.x < 2) counters[threadIdx.x] = 0;
+  if (threadIdx.x < 3) counters[threadIdx.x] = 0;  // (and the gate)
   if (p.far_segs == 0) return;
   __shared__ int n_listed;
   if (threadIdx.x == 0) n_listed = 0;

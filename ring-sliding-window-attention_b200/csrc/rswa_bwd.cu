@@ -135,8 +135,9 @@ rswa_bwd_kernel(const __grid_constant__ BwdKernelParams p, int n_tile_items) {
     tmem_alloc(&ctl->tmem_base, kBwdTmemCols);
     tmem_relinquish();
   }
-  // (behind the wait, not in front of it: the dQ kernel relies on the delta kernel having finished)
+  // (the trigger behind the wait: an overlapping dQ kernel relies on all that came before this one)
   griddep_wait();
+  if (p.gate != nullptr && blockIdx.x == 0 && threadIdx.x == 0) gate_open(p.gate);
   griddep_launch();
   if (threadIdx.x == 0) ctl->err = (smem_u32(smem) & 1023u) ? 199 : status_code(p.status, p.mirror);
   tc_fence_before();

@@ -78,6 +78,7 @@ struct BwdKernelParams {
   void* dq;  // [batch, q_len, hq, 128], 16-bit, written by the dQ kernel
   int* dq_counter;   // work counter of the dQ kernel, zeroed before its launch
   int* dkv_counter;  // work counter of the dK/dV kernel, likewise
+  int* gate;         // 0 until the dK/dV kernel hands what came before it on to an overlapping dQ kernel; null: no overlap
   long long dq_sb, dq_st, dq_sh;
   int* status;
   int* mirror;  // host-visible copy of the status word (or null)
@@ -96,7 +97,10 @@ struct BwdKernelParams {
 // kernel has finished and its writes are visible (at once if the kernel was launched the ordinary way),
 // griddep_launch() says that the next kernel may be brought up as far as SMs are free (without it that is when
 // the kernel ends: the launch itself is hidden then).  Nothing may be read from or written to global memory in
-// front of griddep_wait(), with one exception that the dQ kernel explains.
+// front of griddep_wait(), with one exception: the dQ kernel, which overlaps the dK/dV kernel in front of it and needs what
+// the kernels before THAT one wrote.  Starting behind its trigger promises no visibility (only griddep_wait() does, to
+// the grid that waits), so the dK/dV kernel passes on what its own wait has made visible: tc05::gate_open() releases
+// a word, tc05::gate_wait() acquires it.  (One load of a few hundred ns per dQ CTA, behind the barrier set-up.)
 // Measured, one GPU: training step of 4096 tokens (32/4 heads, window 1000) 319 -> 290 us, prefill of 777 tokens
 // 17.4 -> 15.4 us, 65536 tokens with 32/32 heads 5796 -> 5795 us.  A griddep_launch() in the forward kernel with
 // an early delta kernel behind it made the large calls 1.5 to 5 % slower and gave the small ones nothing.

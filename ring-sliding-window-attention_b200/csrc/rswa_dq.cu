@@ -127,11 +127,12 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
     mbar_init(&ctl->ds_ready, kDqCompute / 32);  // one arrival per compute warp
     mbar_init(&ctl->done, 1);
     mbar_init(&ctl->dq_drained, kDqCompute / 32);  // one arrival per compute warp
-    // No griddep_wait() here: when this kernel starts early, the kernel it overlaps is the dK/dV kernel of the same
-    // call, which it needs nothing from and which lets it start only after the delta kernel, and with it everything
-    // that came before the call, has finished.  The wait is at the end instead.
-    ctl->err = (smem_u32(smem) & 1023u) ? 199 : status_code(p.status, p.mirror);
     mbar_fence_init();
+    // No griddep_wait() here: when this kernel starts early, the kernel it overlaps is the dK/dV kernel of the same
+    // call, which it needs nothing from.  What the delta kernel and everything before the call wrote comes through the
+    // gate: acquired here, by the other threads through the barrier below.  The wait is at the end instead.
+    const bool open = p.gate == nullptr || gate_wait(p.gate);
+    ctl->err = (smem_u32(smem) & 1023u) ? 199 : !open ? kErrWaitProducer : status_code(p.status, p.mirror);
   }
   if (warp == 1) {
     tmem_alloc(&ctl->tmem_base, kDqTmemCols);
@@ -155,6 +156,7 @@ rswa_dq_kernel(const __grid_constant__ BwdKernelParams p, int n_q_tiles, int n_i
       // ------------------------------------------------------------------ key-tile lists + TMA producer
       // One loop turn per key tile and ONE copy of each load's code (this thread runs through its code
       // at the pace of instruction fetch, and the kernel has to fit the instruction cache).
+      if (p.gate != nullptr) fence_proxy_async_global();  // what came through the gate is read by TMA here
       int n = -1, kc = 0, ic = 0;  // item of this CTA, K/V tiles loaded so far, items with work so far
       int j = 0, n_tiles = 0, slot = 0;
       DqItem w = {};

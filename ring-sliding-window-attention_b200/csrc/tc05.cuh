@@ -81,8 +81,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// A word through which one kernel hands on to another what it has seen written (see griddep_wait).
+__device__ __forceinline__ void gate_open(int* gate) { asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(gate) : "memory"); }
+// false: not opened in time (limited like every wait; an overlapping kernel starts behind the trigger of all CTAs of the
+// one that opens the gate, so that all it can have to wait for is a store on its way)
+__device__ __forceinline__ bool gate_wait(const int* gate) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0; i < RSWA_SPIN_LIMIT; ++i) {
+    int open;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(open) : "l"(gate) : "memory");
+    if (open != 0) return true;
+    __nanosleep(100);
+    uint64_t now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (t0 == 0) t0 = now;
+    else if (now - t0 > RSWA_WAIT_LIMIT_NS) break;
+  }
+  return false;
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- TMA (no multicast)
