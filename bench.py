@@ -404,6 +404,40 @@ def time_streaming_kernels(K, q, do, steps):
     return merge_ms, merge_bytes, delta_ms, delta_bytes
 
 
+def time_steps(K, one_step, steps, sync_all):
+    """(milliseconds, kernels of this library launched) of `steps` steps the way a program makes them: no events
+    inside, which would send single-GPU calls down another host path and keep the backward's kernels apart."""
+    launches0 = K.launch_count
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    sync_all()
+    e0.record()
+    for _ in range(steps):
+        one_step()
+    e1.record()
+    sync_all()
+    return e0.elapsed_time(e1), K.launch_count - launches0
+
+
+def time_kernels(K, one_step, steps, sync_all):
+    """Milliseconds per step of the forward, dK/dV and dQ kernels, from a pass of its own with events around each
+    (the backward's two run one after the other in it, where an ordinary step overlaps them)."""
+    from ring_swa import _C
+    lib = _C.lib()
+    K.fwd_events, K.bwd_main_events = fwd, bwd = [], []
+    try:
+        for _ in range(steps):
+            one_step()
+        sync_all()
+    finally:
+        K.fwd_events = K.bwd_main_events = None
+    ms = (sum(lib.rswa_event_elapsed_ms(a, b) for a, b in fwd) / steps,
+          sum(lib.rswa_event_elapsed_ms(a, m) for a, m, _ in bwd) / steps, sum(lib.rswa_event_elapsed_ms(m, b) for _, m, b in bwd) / steps)
+    for events in fwd + bwd:
+        for e in events:
+            lib.rswa_event_destroy(e)
+    return ms
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -441,7 +475,6 @@ def main():
         group = dist.group.WORLD
 
     import ring_swa
-    from ring_swa import _C
     from ring_swa import _kernels as K
 
     fn = getattr(ring_swa, wl["fn"])
@@ -491,29 +524,14 @@ def main():
     if sampler:
         sampler.start()
         time.sleep(0.3)
-    K.fwd_events, K.bwd_main_events = [], []
-    launches0 = K.launch_count
-    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     sync_all()
     if sampler:
         sampler.mark()
-    e0.record()
-    for _ in range(args.steps):
-        step(q, k, v, do)
-    e1.record()
-    sync_all()
+    ms, launches = time_steps(K, lambda: step(q, k, v, do), args.steps, sync_all)
     if sampler:
         sampler.mark()
-    ms = e0.elapsed_time(e1)
-    launches = K.launch_count - launches0
-    lib = _C.lib()
-    fwd_ms = sum(lib.rswa_event_elapsed_ms(a, b) for a, b in K.fwd_events) / args.steps
-    bwd_ms = sum(lib.rswa_event_elapsed_ms(a, m) for a, m, b in K.bwd_main_events) / args.steps     # dK/dV kernel
-    dq_ms = sum(lib.rswa_event_elapsed_ms(m, b) for a, m, b in K.bwd_main_events) / args.steps      # dQ kernel
-    for evs in K.fwd_events + K.bwd_main_events:
-        for e in evs:
-            lib.rswa_event_destroy(e)
-    K.fwd_events = K.bwd_main_events = None
+    time.sleep(0.3)     # as in front of the timed region: a loop without a pause reaches the power cap, and lower clocks
+    fwd_ms, bwd_ms, dq_ms = time_kernels(K, lambda: step(q, k, v, do), args.steps, sync_all)
     K.check_device_status(dev)
 
     # ---------------------------------------------------------------- end to end (host buffers)
@@ -682,7 +700,8 @@ def main():
             "roofline": {"kernel": "rswa_bwd_kernel (dK/dV)", "bound": "tensor", "achieved": ach_bwd, "peak": peak_tf,
                          "unit": "TFLOP/s", "frac": ach_bwd / peak_tf, "traffic": TRAFFIC_DKDV_CFG2 if args.workload == "cfg2" and n == 1 else None,
                          "peak_source": f"{peak_kind} {peak_name}", "ms_per_launch": bwd_ms,
-                         "algorithmic_flops_per_launch": flops_bwd},
+                         "algorithmic_flops_per_launch": flops_bwd,
+                         "timed": "the three kernels' times: a pass of their own, an event around each, one after the other; value: without events"},
             "roofline_dq": {"kernel": "rswa_dq_kernel", "bound": "tensor", "achieved": ach_dq, "peak": peak_tf,
                             "unit": "TFLOP/s", "frac": ach_dq / peak_tf, "ms_per_launch": dq_ms,
                             "algorithmic_flops_per_launch": flops_dq},

@@ -621,3 +621,23 @@ def test_sink_gradients_of_more_than_65535_rows():
     x = [torch.randn(8, 385, 1, 64, device="cuda").bfloat16().repeat(8192, 1, 1, 1) for _ in range(4)]
     for t in _grads(lambda q, k, v: ring_swa.ring_streaming_llm_attn(q, k, v, 60), x[:3], x[3]):
         assert torch.equal(t[:8], t[-8:])
+
+
+def test_benchmark_times_the_path_of_ordinary_calls():
+    """Event lists send single-GPU calls down another host path and keep the backward's kernels apart: the
+    benchmark's step time is taken without them, the kernels' times in a pass of their own."""
+    import bench
+    from ring_swa import _kernels as K
+    import ring_swa
+    x = [randn_bf16(1, 300, h, D, seed=30 + i).cuda() for i, h in enumerate((4, 2, 2))]
+    do = randn_bf16(1, 300, 4, D, seed=33).cuda()
+    events = []
+
+    def step():
+        events.append((K.fwd_events, K.bwd_main_events))
+        _grads(lambda *t: ring_swa.ring_sliding_window_attn(*t, 100), x, do)
+
+    ms, launches = bench.time_steps(K, step, 3, torch.cuda.synchronize)
+    assert events == [(None, None)] * 3 and ms > 0 and launches == 3 * 4   # forward, delta, dK/dV, dQ
+    assert all(t > 0 for t in bench.time_kernels(K, step, 2, torch.cuda.synchronize))
+    assert None not in events[3] and K.fwd_events is None and K.bwd_main_events is None
