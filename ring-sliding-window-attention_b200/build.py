@@ -17,6 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "ring_swa", "librswa.so")
 NATIVE_OUT = os.path.join(HERE, "ring_swa", "_native.so")
+NATIVE_STAMP = NATIVE_OUT + ".stamp"
 NATIVE_SOURCE = os.path.join(CSRC, "rswa_torch.cpp")
 SOURCES = ["rswa_api.cu", "rswa_fwd.cu", "rswa_bwd.cu", "rswa_dq.cu", "rswa_aux.cu", "rswa_selftest.cu", "rswa_noalloc.cu", "rswa_peer.cu"]
 HEADERS = ["tc05.cuh", "rswa_common.cuh", "rswa_tiles.cuh", os.path.join("..", "..", "include", "rswa.h")]
@@ -41,10 +42,25 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def _native_abi() -> str:
+    """What _native.so is bound to besides its source: it includes torch's and Python's headers."""
+    import torch
+    return f"torch {torch.__version__} cxx11 {int(torch._C._GLIBCXX_USE_CXX11_ABI)} {sys.implementation.cache_tag}"
+
+
+def native_is_stale() -> bool:
+    if not os.path.exists(NATIVE_OUT) or not os.path.exists(NATIVE_STAMP):
+        return True
+    with open(NATIVE_STAMP) as f:
+        if f.read() != _native_abi():
+            return True
+    deps = [NATIVE_SOURCE, os.path.join(CSRC, "..", "..", "include", "rswa.h"), os.path.abspath(__file__)]
+    return os.path.getmtime(NATIVE_OUT) <= max(os.path.getmtime(d) for d in deps)
+
+
 def build_native(force: bool = False) -> str:
     """The torch-facing host path; needs librswa.so, whose directory it looks in at load time."""
-    deps = [NATIVE_SOURCE, os.path.join(CSRC, "..", "..", "include", "rswa.h"), os.path.abspath(__file__)]
-    if not force and os.path.exists(NATIVE_OUT) and os.path.getmtime(NATIVE_OUT) > max(os.path.getmtime(d) for d in deps):
+    if not force and not native_is_stale():
         return NATIVE_OUT
     import torch
     root = os.path.dirname(torch.__file__)
@@ -58,6 +74,8 @@ def build_native(force: bool = False) -> str:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(_native_abi())
     return NATIVE_OUT
 
 

@@ -79,3 +79,16 @@ def test_product_has_no_cpu_path():
     q = torch.zeros(1, 128, 2, 128, dtype=torch.bfloat16)
     with pytest.raises(RuntimeError, match="no CPU path"):
         ring_swa.ring_sliding_window_attn(q, q, q, 10)
+
+
+def test_native_module_is_rebuilt_for_another_torch(monkeypatch):
+    """_native.so includes torch's headers: the file of another version is stale whatever its time."""
+    import importlib.util
+    import torch
+    spec = importlib.util.spec_from_file_location("rswa_build", os.path.join(ROOT, "ring-sliding-window-attention_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    build.build()
+    assert not build.native_is_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.native_is_stale()
