@@ -545,7 +545,6 @@ rswa_fwd_kernel(const __grid_constant__ FwdKernelParams p, int n_blocks, int n_i
           lacc = make_float2(0.f, 0.f);
           exps(r[0], tS);
           exps(r[1], tS + 16);
-          if (!ok) break;
           RSWA_TRC(fwd, lane == 0 && quad == 0 && n == RSWA_TRACE_ITEM && j < 32, j * 32 + 12 + 8 * w);
           // The first kPSplit k-steps of P (96 keys) are handed over when they are complete, so that their share of
           // O_w += P_w V runs while the last 32 exponentials of the row are computed.
