@@ -235,8 +235,10 @@ int sm_count() {
 // 1000 that chain of 1000 tile products was 1.7 of the kernel's 1.75 ms.  The queries beyond the window are cut
 // into segments instead, each about as long as an ordinary key tile's item (`per_key` query tiles), so that no
 // item is longer than the others.  Left alone: calls short enough for the chain to be at most twice an
-// ordinary item (the partial sums cost another launch), very many sink tokens (the partial sums are kept per
-// sink token) and packs of sequences shorter than a tile on average (their segments would be mostly empty).
+// ordinary item (the partial sums cost another launch); more than 16 sink tokens, for the memory: the partial sums are
+// kept per sink token and are about as large as q for 16 of them in a pack of sequences of one tile (4096
+// tokens, 32/8 heads, window 256, 17 sink tokens: 310 us a training step where segments would take 218; from 16384
+// tokens on the two differ by less than 1 %); and packs of sequences shorter than a tile on average.
 struct FarPlan {
   int segs, chunk, slots;
   int64_t sum_bytes, bytes;  // partial sums; with the list of segments behind them

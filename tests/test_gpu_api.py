@@ -80,7 +80,7 @@ def test_varlen_functions():
 
 def test_device_side_timeout_reaches_the_host_and_clears():
     """A bounded device-side wait that runs out raises the status word; kernels launched after that do no
-    work, so the host has to hear of it: the word is mirrored to pinned memory behind every backward and
+    work, so the host has to hear of it: a kernel that finds the word raised also writes it to pinned memory, which is
     looked at when the next call starts.  The word is set from the host here (nothing on the device
     faults or waits)."""
     import ring_swa
@@ -105,8 +105,8 @@ def test_device_side_timeout_reaches_the_host_and_clears():
 @pytest.mark.parametrize("head_dim", [64, 96])
 def test_smaller_head_dims_run_zero_padded(head_dim):
     """Head dimensions below 128 (the reference's own local tests use 1 x 1024 x 8/2 heads x 64, window 128:
-    test/test_local_slm.py:76-90) run on the 128-wide kernels zero-padded; result and gradients have the
-    caller's shape and match the oracle at the caller's scale."""
+    test/test_local_slm.py:76-90) run on the 128-wide kernels zero-padded (64 across several GPUs or with events; alone
+    it has kernels of its own); result and gradients have the caller's shape and match the oracle at the caller's scale."""
     import ring_swa
     q, k, v, do = (randn_bf16(1, 1024, h, head_dim, seed=s) for h, s in ((8, 71), (2, 72), (2, 73), (8, 74)))
     for fn, ns in ((ring_swa.ring_sliding_window_attn, 0), (ring_swa.ring_streaming_llm_attn, 1)):
@@ -641,3 +641,71 @@ def test_benchmark_times_the_path_of_ordinary_calls():
     assert events == [(None, None)] * 3 and ms > 0 and launches == 3 * 4   # forward, delta, dK/dV, dQ
     assert all(t > 0 for t in bench.time_kernels(K, step, 2, torch.cuda.synchronize))
     assert None not in events[3] and K.fwd_events is None and K.bwd_main_events is None
+
+
+def test_64_wide_heads_zero_padded():
+    """Heads of 64 elements on the path of calls across several GPUs."""
+    from ring_swa import _ring
+    q, k, v, do = (randn_bf16(1, 700, h, 64, seed=s) for h, s in ((8, 71), (2, 72), (2, 73), (8, 74)))
+    ro, _, rdq, rdk, rdv = dense_attn_fwd_bwd(q, k, v, do, 128, None, 1)
+    ring = _ring.ring_ctx(None, None, None, None, None)
+    got = _run(lambda *x: _ring.attention(*x, 128, 1, None, None, None, ring), q, k, v, do)
+    for n, a, b in zip(("out", "dq", "dk", "dv"), got, (ro, rdq, rdk, rdv)):
+        assert_close(n, a, b)
+
+
+@pytest.mark.parametrize("n_sink", [0, 1])
+def test_captured_training_step(n_sink):
+    """A public function and its backward inside a CUDA graph: replays on new values of the same tensors."""
+    import ring_swa
+    x, x2 = ([randn_bf16(1, 1200, h, D, seed=seed + i).cuda() for i, h in enumerate((4, 2, 2, 4))] for seed in (30, 60))
+
+    def fn(q, k, v):
+        return ring_swa.ring_streaming_llm_attn(q, k, v, 100) if n_sink else ring_swa.ring_sliding_window_attn(q, k, v, 100)
+
+    static = [t.clone() for t in x]
+    _grads(fn, static[:3], static[3])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _grads(fn, static[:3], static[3])
+    for values in (x2, x):
+        for s, t in zip(static, values):
+            s.copy_(t)
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, _grads(fn, values[:3], values[3])))
+
+
+def test_sink_gradients_of_a_long_sequence_against_64_bits():
+    """32768 tokens: the gradients of the sink tokens, sums over every query, in float32 buffers.  A term (P x dO or
+    dS x q) is rounded once, to 2^-9 of its size at most, and its rounding is independent of the next one's: with terms of
+    random sign the sum's error stays below 2^-9 of the sum, in norm; dS also carries the rounding of `out`,
+    as much again.  Summed in segments it is no further off than in one chain over all queries (the two share
+    the terms, whose error is nearly all of it)."""
+    from ring_swa import _kernels as K
+    S, W, n_sink, Hq, scale = 32768, 1000, 4, 4, D ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(1, S, h, D, device="cuda", generator=g).bfloat16() for h in (Hq, 1, 1, Hq))
+    kd, vd = k[0, :, 0].double(), v[0, :, 0].double()
+    rdk, rdv = torch.zeros(n_sink, D, dtype=torch.float64, device="cuda"), torch.zeros(n_sink, D, dtype=torch.float64, device="cuda")
+    for c0 in range(0, S, 4096):
+        keys = torch.arange(max(0, c0 - W), c0 + 4096, device="cuda")
+        keys = torch.cat([torch.arange(n_sink, device="cuda"), keys[keys >= n_sink]])
+        pos = torch.arange(c0, c0 + 4096, device="cuda")[:, None]
+        seen = (keys <= pos) & ((pos - keys <= W) | (keys < n_sink))
+        for h in range(Hq):
+            qd, dod = q[0, c0:c0 + 4096, h].double(), do[0, c0:c0 + 4096, h].double()
+            p = torch.softmax((qd @ kd[keys].T * scale).masked_fill(~seen, float("-inf")), -1)
+            delta = (p @ vd[keys] * dod).sum(-1, keepdim=True)
+            ds = p[:, :n_sink] * (dod @ vd[:n_sink].T - delta)
+            rdk += ds.T @ qd * scale
+            rdv += p[:, :n_sink].T @ dod
+    out, lse = K.fwd(q, [K.KVSpan(k, v, 0)], W, n_sink, scale)
+    err = []
+    for ws in (None, K.bwd_workspace(q)):      # in segments, in one chain
+        dk, dv = (torch.empty(k.shape, dtype=torch.float32, device="cuda") for _ in range(2))
+        K.bwd(q, [K.KVSpan(k, v, 0, dk=dk, dv=dv)], out, lse, do, torch.empty_like(q), W, n_sink, scale, workspace=ws)
+        err.append([float((a[0, :n_sink, 0].double() - r).norm() / r.norm()) for a, r in ((dk, rdk), (dv, rdv))])
+    K.check_device_status()
+    (dk_seg, dv_seg), (dk_chain, dv_chain) = err
+    assert dv_seg <= 2 ** -9 and dk_seg <= 2 * 2 ** -9
+    assert dv_seg <= 1.02 * dv_chain and dk_seg <= 1.02 * dk_chain
