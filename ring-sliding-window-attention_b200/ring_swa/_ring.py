@@ -391,11 +391,11 @@ def ring_ctx(cp_group, cp_size, cp_local_rank, cp_prev_global_rank, cp_next_glob
 
 
 def single_gpu(q, k, v, window_size: int, n_sink: int, softmax_scale: Optional[float], cu_seqlens):
-    """A call without a group, autograd included, in C++ (csrc/rswa_torch.cpp): one training step of its two
-    halves costs the host 20 us next to the autograd engine's own, 200 through RingAttn.  The public functions try
-    it before anything else; it returns None for what it leaves to the code below -- arguments that do not
-    fit together, other dtypes or devices, an error of an earlier call to report -- and when events, NVTX
-    ranges or plans are to be recorded, which only that code does."""
+    """A call without a group, autograd included, in C++ (csrc/rswa_torch.cpp, with the host times of both paths).
+    The public functions try it before anything else; it returns None for what it leaves to the code below --
+    arguments that do not fit together, other dtypes, devices or tensor types, traces and transforms, an error
+    of an earlier call to report -- and when events, NVTX ranges or plans are to be recorded, which only that
+    code does."""
     if _NVTX or _DEBUG or _phase_events is not None or K.fwd_events is not None or K.bwd_main_events is not None:
         return None
     return _native_attention(q, k, v, window_size, n_sink, softmax_scale, cu_seqlens)
