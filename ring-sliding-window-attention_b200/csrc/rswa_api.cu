@@ -12,8 +12,8 @@ namespace rswa {
 int launch_fwd(const FwdKernelParams& kp, int dtype, cudaStream_t stream);
 int launch_bwd(const BwdKernelParams& kp, int dtype, int total_key_tiles, bool early, cudaStream_t stream);
 int launch_sink_sum(const BwdKernelParams& kp, int dtype, cudaStream_t stream);
-int launch_begin_call(const BwdKernelParams& next, int* counters, cudaStream_t stream);
-int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, const BwdKernelParams& next, int* counters,
+int launch_begin_call(const FarParams& far, int* counters, cudaStream_t stream);
+int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, const FarParams& far, int* counters,
                  cudaStream_t stream);
 int launch_dq(const BwdKernelParams& kp, int dtype, bool early, cudaStream_t stream);
 
@@ -472,7 +472,8 @@ static int bwd_call(const rswa_bwd_params_t* p, int head_dim, void* stream_) {
   }
 
   // (both kernels also reset the work counters and list the segments)
-  rc = (p->flags & RSWA_BWD_INIT) ? launch_delta(*p, delta, lse2, q_len_pad, kk, dq_counter, stream) : launch_begin_call(kk, dq_counter, stream);
+  const FarParams fp = {kk.cu, kk.n_seqs, kk.q_pos_start, kk.q_len, kk.window, kk.far_segs, kk.far_chunk, kk.far_list};
+  rc = (p->flags & RSWA_BWD_INIT) ? launch_delta(*p, delta, lse2, q_len_pad, fp, dq_counter, stream) : launch_begin_call(fp, dq_counter, stream);
   if (rc) return rc;
   // The two tensor kernels overlap: the dQ kernel takes over the SMs that the dK/dV kernel runs out of work for
   // (20 of 148 have none from the start, at 4096 tokens of 32/4 heads).  Not where an event between the two is asked

@@ -35,7 +35,7 @@ __device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
 // Without the list the kernel's CTAs drew every segment from the work counter and dropped those without work, at
 // 1.5 us each: 65536 tokens in 400 sequences, 32/8 heads, window 1000 (no sequence reaches beyond it): 2114 us a training
 // step, 2084 with the list, 2077 without anything for sink tokens.
-__device__ __forceinline__ void begin_call(const BwdKernelParams& p, int* counters) {
+__device__ __forceinline__ void begin_call(const FarParams& p, int* counters) {
   if (threadIdx.x < 3) counters[threadIdx.x] = 0;  // (and the gate)
   if (p.far_segs == 0) return;
   __shared__ int n_listed;
@@ -51,8 +51,8 @@ __device__ __forceinline__ void begin_call(const BwdKernelParams& p, int* counte
   __syncthreads();
   if (threadIdx.x == 0) p.far_list[0] = n_listed;
 }
-__global__ void __launch_bounds__(256) begin_call_kernel(const __grid_constant__ BwdKernelParams next, int* counters) {
-  begin_call(next, counters);
+__global__ void __launch_bounds__(256) begin_call_kernel(FarParams far, int* counters) {
+  begin_call(far, counters);
 }
 
 // A warp takes 32 consecutive tokens of one (batch row, head): 16 lanes per 128-element row (16 bytes per lane and
@@ -65,9 +65,9 @@ __global__ void delta_kernel(const uint16_t* __restrict__ out, long long o_sb, l
                              const uint16_t* __restrict__ dout, long long d_sb, long long d_st, long long d_sh,
                              const float* __restrict__ lse, long long l_sb, long long l_sh,
                              float* __restrict__ delta, float* __restrict__ lse2, int batch, int q_len, int hq,
-                             int q_len_pad, const __grid_constant__ BwdKernelParams next, int* counters) {
+                             int q_len_pad, FarParams far, int* counters) {
   griddep_launch();  // (to the dK/dV kernel, which waits for this one)
-  if (blockIdx.x == 0) begin_call(next, counters);
+  if (blockIdx.x == 0) begin_call(far, counters);
   const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // warp task
   const int lane = threadIdx.x & 31;
   constexpr int kLanes = kD / 8, kRows = 32 / kLanes;  // lanes per row, rows per load
@@ -355,13 +355,12 @@ int check_launch(const char* what) {
 
 }  // namespace
 
-// next: the call's dK/dV kernel
-int launch_begin_call(const BwdKernelParams& next, int* counters, cudaStream_t stream) {
-  begin_call_kernel<<<1, 256, 0, stream>>>(next, counters);
+int launch_begin_call(const FarParams& far, int* counters, cudaStream_t stream) {
+  begin_call_kernel<<<1, 256, 0, stream>>>(far, counters);
   return check_launch("rswa_bwd(begin)");
 }
 
-int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, const BwdKernelParams& next, int* counters,
+int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_len_pad, const FarParams& far, int* counters,
                  cudaStream_t stream) {
   const rswa_geom_t& g = p.g;
   const long long tasks = static_cast<long long>(g.batch) * g.n_q_heads * (q_len_pad / 32);  // one warp each
@@ -373,7 +372,7 @@ int launch_delta(const rswa_bwd_params_t& p, float* delta, float* lse2, int q_le
   kern<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(
       static_cast<const uint16_t*>(p.out), p.o_stride_b, p.o_stride_t, p.o_stride_h,
       static_cast<const uint16_t*>(p.dout), p.do_stride_b, p.do_stride_t, p.do_stride_h, p.lse, p.lse_stride_b,
-      p.lse_stride_h, delta, lse2, g.batch, g.q_len, g.n_q_heads, q_len_pad, next, counters);
+      p.lse_stride_h, delta, lse2, g.batch, g.q_len, g.n_q_heads, q_len_pad, far, counters);
   return check_launch("rswa_bwd(delta)");
 }
 

@@ -92,6 +92,13 @@ struct BwdKernelParams {
   int* far_list;  // number of segments that are work items, then these segments (written by begin_call)
 };
 
+// What the kernel in front of the tensor kernels needs of these (the whole struct is 3 KB of tensor maps).
+struct FarParams {
+  const int* cu;
+  int n_seqs, q_pos_start, q_len, window, far_segs, far_chunk;
+  int* far_list;
+};
+
 // Programmatic dependent launch.  The tensor kernels are launched with the attribute that lets a kernel start while
 // the one before it on the stream still runs (launch_kernel below): griddep_wait() returns once every earlier
 // kernel has finished and its writes are visible (at once if the kernel was launched the ordinary way),
@@ -143,7 +150,8 @@ __device__ __forceinline__ int seq_of(const int* __restrict__ cu, int n_seqs, in
 // segment e lies in one sequence and one chunk.  With i sequence starts and j chunk boundaries in front of
 // it, e = i + j and it belongs to sequence i.  Fills the sequence's bounds and the positions [q_lo, q_hi] of the
 // segment's queries that lie beyond the window of the sequence's first token (none if q_lo > q_hi).
-__device__ __forceinline__ void far_range(const BwdKernelParams& p, int i, int j, int& s, int& e, int& q_lo, int& q_hi) {
+template <typename Params>
+__device__ __forceinline__ void far_range(const Params& p, int i, int j, int& s, int& e, int& q_lo, int& q_hi) {
   s = 0, e = 0x7fffffff;
   if (p.cu != nullptr) {
     s = __ldg(p.cu + i);
@@ -160,13 +168,15 @@ __device__ __forceinline__ void far_range(const BwdKernelParams& p, int i, int j
 // than one segment.  Fewer cost the sink tokens' key tile at most as many tile products again as an ordinary one has,
 // and a segment item (its loads, its partial sums) costs more: 32768 tokens in 250 sequences of 131, 32/8
 // heads, window 64, 4 sink tokens: 1086 us a training step without segments, 1280 us with one for each sequence.
-__device__ __forceinline__ bool far_split(const BwdKernelParams& p, int s, int e) {
+template <typename Params>
+__device__ __forceinline__ bool far_split(const Params& p, int s, int e) {
   if (p.far_segs == 0) return false;
   const int first = s > 0x7ffffffe - p.window ? 0x7fffffff : s + p.window + 1;
   return min(e, p.q_pos_start + p.q_len) - max(first, p.q_pos_start) > p.far_chunk;
 }
 // number of sequence starts among the first e of the merged boundaries (starts first on ties)
-__device__ __forceinline__ int far_sequence(const BwdKernelParams& p, int e) {
+template <typename Params>
+__device__ __forceinline__ int far_sequence(const Params& p, int e) {
   if (p.cu == nullptr) return 0;
   const int n_b = (p.q_len + p.far_chunk - 1) / p.far_chunk - 1;  // boundary j at q_pos_start + (j + 1) * far_chunk
   int lo = max(0, e - n_b), hi = min(e, p.n_seqs);                // start i at cu[i + 1]
